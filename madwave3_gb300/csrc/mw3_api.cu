@@ -202,6 +202,7 @@ int build_device(Ctx &c)
         return MW3_ERR_STATE;
     }
     free_device(c);
+    c.fl_pending = c.cv_pending = false;
     int na = c.na, n1 = c.n1, n2 = c.n2, ne = c.ne;
     int W = (int)c.waves.size();
     c.ang_cw = c.k_cw > 0 ? c.k_cw : c.ang_cw_fit;
@@ -878,6 +879,7 @@ int check_device_flags(Ctx &c, const char *where)
 
 int reset_accumulators(Ctx &c)
 {
+    c.fl_pending = c.cv_pending = false;
     size_t nf = (size_t)std::max(c.NF, 1) * c.netot * 2;
     if (c.d_cvcring)
         MW3_CUDA_TRY(cudaMemsetAsync(c.d_cvcring, 0, sizeof(float) * mw3::kFluxRing * c.netot * 2, c.stream));
@@ -1218,6 +1220,7 @@ int mw3_run(mw3_ctx *h, int64_t n)
         for (size_t i = old; i < c.prof_ev.size(); i++) MW3_CUDA_TRY(cudaEventCreate(&c.prof_ev[i]));
         c.prof_cap = need;
     }
+    if (n > 0) c.fl_pending = c.cv_pending = true;
     for (int64_t s = 0; s < n;) {
         if (graph_ready(c, n - s)) {
             // kGraphIters iterations as one graph replay
@@ -1353,8 +1356,9 @@ int mw3_totalflux(mw3_ctx *h, int32_t w, double *tot, double *elec)
     double *d = nullptr;
     mw3::flush_flux(c);
     mw3::flush_cvj(c);
-    MW3_CUDA_TRY(cudaMallocAsync(&d, sizeof(double) * (size_t)t.netot * (1 + c.ne), c.stream));
-    mw3::launch_totalflux(c, w, d, d + t.netot);
+    const size_t row = (size_t)t.netot * (1 + c.ne);        // P(E), then each state's
+    MW3_CUDA_TRY(cudaMallocAsync(&d, sizeof(double) * row * (1 + mw3::totalflux_chunks(c, w)), c.stream));
+    mw3::launch_totalflux(c, w, d + row, d);
     MW3_CUDA_TRY(cudaMemcpyAsync(tot, d, sizeof(double) * t.netot, cudaMemcpyDeviceToHost, c.stream));
     if (elec)
         MW3_CUDA_TRY(cudaMemcpyAsync(elec, d + t.netot, sizeof(double) * (size_t)t.netot * c.ne,

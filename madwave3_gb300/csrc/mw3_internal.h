@@ -262,6 +262,9 @@ struct Ctx {
     int4 *d_fl_runs = nullptr;       // (flat index lo, flat index hi, first r1, length)
     bool fl_runs = false;
     float *d_cring = nullptr;        // [kFluxSlots][netot][2]
+    // iterations since the rings were last added in full: without any, reading the
+    // accumulators need not add the (cleared) rings again
+    bool fl_pending = false, cv_pending = false;
     int fl_q = 32;                   // a slice of the flux points is flushed every fl_q iterations
     // mixed path: the Cvj projection in FP32 (from the FP32 copy of psi) and Cvj of the
     // last kFluxRing iterations with their C_k(E) (slot = iteration mod kFluxRing),
@@ -425,7 +428,8 @@ constexpr int kGraphIters = 32;      // iterations per captured graph (one ring 
 static_assert(kFluxRing == kGraphIters, "a captured block must cycle the Cvj ring exactly once");
 static_assert(kGraphIters % (kFluxSlots / 4) == 0, "flux slice flushes must repeat with the captured block");
 void launch_addv(Ctx &c, const double *psi, int g0, int g1);
-void launch_totalflux(Ctx &c, int w, double *d_out, double *d_outelec);
+int totalflux_chunks(const Ctx &c, int w);
+void launch_totalflux(Ctx &c, int w, double *d_part, double *d_out);
 void set_kernel_attributes(Ctx &c);
 // picks c.ang_cw so that every kernel's dynamic shared memory fits optin bytes
 bool fit_smem(Ctx &c, size_t optin);

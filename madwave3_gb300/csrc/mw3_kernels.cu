@@ -1433,27 +1433,65 @@ __global__ void __launch_bounds__(256) k_cvj_acc(DevGrid d, CvjArgs c)
     c.zs2[2 * e + 1] += z * c.zck[2 * ie + 1];
 }
 
-// totalflux (mod_flux_01y2.f:778-816) for one wave's flux points
-__global__ void k_totalflux(const double *__restrict__ zcr, const double *__restrict__ zcdr,
-                            const int *__restrict__ fblock, const int *__restrict__ nelebas, int nflux, int netot,
-                            int nelec, const double *__restrict__ reacfct, double ah1, double *__restrict__ out,
-                            double *__restrict__ outelec)
+// totalflux (mod_flux_01y2.f:778-816) for one wave's flux points, in two passes:
+// part[c][0][E] = sum over the flux points of chunk c of Im(conj(zCR) zCdR), and
+// part[c][1 + e][E] its share of electronic state e; then the chunks in order.
+// Bound by the read of the accumulators (32 B per point and energy).  One thread
+// an energy over all points left 8 CTAs walking up to tens of thousands of points
+// in a serial chain of loads (J = 10, 25 k points x 1000 energies: 16.8 ms); cut
+// into chunks the same read takes 0.2 ms.
+constexpr int kTfMaxE = 8;           // electronic states (mw3_create admits 8)
+__global__ void __launch_bounds__(128) k_totalflux_part(const double *__restrict__ zcr, const double *__restrict__ zcdr,
+                                                        const int *__restrict__ fblock,
+                                                        const int *__restrict__ nelebas, int nflux, int netot,
+                                                        int nelec, int chunk, double *__restrict__ part)
 {
-    int ie = blockIdx.x * blockDim.x + threadIdx.x;
+    const int ie = blockIdx.x * blockDim.x + threadIdx.x;
+    if (ie >= netot) return;
+    const int f0 = blockIdx.y * chunk, f1 = min(nflux, f0 + chunk);
+    double s = 0.0;
+    double se[kTfMaxE];
+#pragma unroll
+    for (int e = 0; e < kTfMaxE; e++) se[e] = 0.0;
+    constexpr int U = 4;                 // points whose loads are in flight together
+    for (int f = f0; f < f1; f += U) {
+        double2 a[U], b[U];
+        int el[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const bool on = f + u < f1;
+            const size_t o = ((size_t)(on ? f + u : f) * netot + ie) * 2;
+            a[u] = *reinterpret_cast<const double2 *>(zcr + o);
+            b[u] = *reinterpret_cast<const double2 *>(zcdr + o);
+            el[u] = on ? nelebas[fblock[f + u]] - 1 : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (el[u] < 0) continue;
+            const double im = a[u].x * b[u].y + (-a[u].y) * b[u].x;
+            s = s + im;
+            if (nelec > 1)
+#pragma unroll
+                for (int e = 0; e < kTfMaxE; e++)
+                    if (el[u] == e) se[e] = se[e] + im;
+        }
+    }
+    double *p = part + (size_t)blockIdx.y * (1 + nelec) * netot + ie;
+    p[0] = s;
+#pragma unroll
+    for (int e = 0; e < kTfMaxE; e++)
+        if (e < nelec) p[(size_t)(1 + e) * netot] = nelec > 1 ? se[e] : s;
+}
+
+__global__ void __launch_bounds__(128) k_totalflux_sum(const double *__restrict__ part, int nchunk, int netot, int nelec,
+                                                       const double *__restrict__ reacfct, double ah1,
+                                                       double *__restrict__ out)
+{
+    const int ie = blockIdx.x * blockDim.x + threadIdx.x;
     if (ie >= netot) return;
     double s = 0.0;
-    double se[8];
-    for (int e = 0; e < 8; e++) se[e] = 0.0;
-    for (int f = 0; f < nflux; f++) {
-        size_t o = ((size_t)f * netot + ie) * 2;
-        double im = zcr[o] * zcdr[o + 1] + (-zcr[o + 1]) * zcdr[o];
-        s = s + im;
-        int el = nelebas[fblock[f]] - 1;
-        if (el < 8) se[el] = se[el] + im;
-    }
-    out[ie] = s * reacfct[ie] / ah1;
-    if (outelec)
-        for (int e = 0; e < nelec && e < 8; e++) outelec[(size_t)e * netot + ie] = se[e] * reacfct[ie] / ah1;
+    for (int c = 0; c < nchunk; c++) s += part[((size_t)c * (1 + nelec) + blockIdx.y) * netot + ie];
+    out[(size_t)blockIdx.y * netot + ie] = s * reacfct[ie] / ah1;
 }
 
 // ---------------------------------------------------------------------------
@@ -1963,7 +2001,8 @@ void launch_product(Ctx &c)
 
 void flush_cvj(Ctx &c)
 {
-    if (!c.d_cvring) return;
+    if (!c.d_cvring || !c.cv_pending) return;
+    c.cv_pending = false;
     // slot = iteration mod 32, flushed whole at the iterations = 31 mod 32: pending
     // are the (now + 1) mod 32 iterations since, the slots (now - s) mod 32 < n
     const int n = (int)((c.it + 1) % kFluxRing);
@@ -1991,7 +2030,8 @@ void build_cvj32(Ctx &c)
 
 void flush_flux(Ctx &c)
 {
-    if (!c.d_fring || c.NF == 0) return;
+    if (!c.d_fring || c.NF == 0 || !c.fl_pending) return;
+    c.fl_pending = false;
     const int P = kFluxSlots / c.fl_q, chunk = (c.NF + P - 1) / P;
     dim3 g((c.NF + kFlushF - 1) / kFlushF, (c.netot + kFlushE - 1) / kFlushE);
     k_flux_flush<<<g, 256, 0, c.stream>>>(c.d_fring, c.d_cring, c.d_fl_poti, c.d_etot, c.netot, c.NF, chunk,
@@ -2127,13 +2167,24 @@ void launch_norms(Ctx &c, int64_t slot)
     LAUNCH_CHECK(c);
 }
 
-void launch_totalflux(Ctx &c, int w, double *d_out, double *d_outelec)
+// chunks of flux points of a wave's P(E): two CTAs of 128 energies an SM (of 152) at the usual
+// 1000 energies, and no chunk below 16 points
+int totalflux_chunks(const Ctx &c, int w)
+{
+    const int nf = c.waves[w].nflux, ec = (c.netot + 127) / 128;
+    return std::max(1, std::min((nf + 15) / 16, std::max(1, 304 / ec)));
+}
+
+void launch_totalflux(Ctx &c, int w, double *d_part, double *d_out)
 {
     WaveTables &t = c.waves[w];
     WaveDev &wd = c.wdev[w];
-    double ah1 = (c.grid.rfin1 - c.grid.rmis1) / (double)(c.n1 - 1);
-    k_totalflux<<<(t.netot + 127) / 128, 128, 0, c.stream>>>(wd.zcr, wd.zcdr, wd.fl_block, wd.nelebas, t.nflux,
-                                                             t.netot, c.ne, wd.reacfct, ah1, d_out, d_outelec);
+    const double ah1 = (c.grid.rfin1 - c.grid.rmis1) / (double)(c.n1 - 1);
+    const int nch = totalflux_chunks(c, w), chunk = std::max(1, (t.nflux + nch - 1) / nch), ec = (t.netot + 127) / 128;
+    k_totalflux_part<<<dim3(ec, nch), 128, 0, c.stream>>>(wd.zcr, wd.zcdr, wd.fl_block, wd.nelebas, t.nflux, t.netot,
+                                                          c.ne, chunk, d_part);
+    LAUNCH_CHECK(c);
+    k_totalflux_sum<<<dim3(ec, 1 + c.ne), 128, 0, c.stream>>>(d_part, nch, t.netot, c.ne, wd.reacfct, ah1, d_out);
     LAUNCH_CHECK(c);
 }
 
