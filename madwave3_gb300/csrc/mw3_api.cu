@@ -152,7 +152,7 @@ int build_typed(Ctx &c)
     }
     // explicit angular matrices (not needed when the factorised contraction runs)
     c.d_xj2 = c.d_xl2p = nullptr;
-    if (c.use_tc_ang) {
+    if (c.use_tc_ang || c.use_fx_ang) {
         mw3::launch_build_kinetic<T>(c);
         return MW3_OK;
     }
@@ -740,6 +740,8 @@ int build_device(Ctx &c)
     mw3::set_kernel_attributes(c);
     TRY(mw3::build_tc_ang(c));
     TRY(mw3::build_tc_dst2d(c));
+    TRY(mw3::build_fx(c));
+    TRY(mw3::build_fx_ang(c));
     c.h32 = c.use_tc_dst2d && c.use_tc_ang;
     c.d_h32 = nullptr;
     c.d_vr32 = nullptr;
@@ -1544,7 +1546,7 @@ int mw3_path_flags(mw3_ctx *h, int32_t *flags)
     *flags = ((mw3::tc_dst_supported(c) || c.use_tc_dst2d) ? MW3_PATH_TC_DST : 0) |
              (c.use_tc_dst2d ? MW3_PATH_TC_DST_FUSED : 0) | (c.use_tc_ang ? MW3_PATH_TC_ANG : 0) |
              ((c.use_tc_dst2d && c.dst_f16) ? MW3_PATH_DST_F16 : 0) | (c.x_t ? MW3_PATH_X_T : 0) |
-             ((c.fp64 && c.d_rd_tw) ? MW3_PATH_RADER : 0);
+             ((c.fp64 && c.d_rd_tw && !c.use_fx) ? MW3_PATH_RADER : 0);
     return MW3_OK;
 }
 
@@ -1713,10 +1715,10 @@ namespace {
 // the same kernels with the same launch shapes
 std::vector<int> path_signature(const Ctx &c)
 {
-    const bool explicit_ang = c.na > 1 && (c.fp64 || !c.use_tc_ang);
+    const bool explicit_ang = c.na > 1 && !c.use_tc_ang && !c.use_fx_ang;
     const bool tc3 = !c.fp64 && !c.use_tc_dst2d && mw3::tc_dst_supported(const_cast<Ctx &>(c));
-    return {(int)c.use_tc_dst2d, c.use_tc_dst2d ? (int)c.dst_f16 : -1, (int)tc3, (int)c.use_tc_ang, (int)c.x_t,
-            (int)(c.fp64 && c.d_rd_tw != nullptr), explicit_ang ? c.ang_cw : 0};
+    return {(int)c.use_tc_dst2d, c.use_tc_dst2d ? (int)c.dst_f16 : -1, (int)tc3, (int)(c.use_tc_ang || c.use_fx_ang), (int)c.x_t,
+            (int)(c.fp64 && c.d_rd_tw != nullptr) + 2 * (int)c.use_fx, explicit_ang ? c.ang_cw : 0};
 }
 
 // time n iterations of the propagation from a synthetic state after the warm-up that
@@ -1763,7 +1765,8 @@ extern "C" int mw3_autotune(mw3_ctx *h, int32_t iterations, int32_t scope, int32
     std::vector<int> dsts{k0[0]}, angs{k0[2]};
     if (scope & MW3_TUNE_FORM) {
         if (c.fp64) {
-            if (c.n2 == 256) dsts = {1, 0};
+            dsts = {-1, 0};              // the digit products, the folded dense ones, Rader where it applies
+            if (c.n2 == 256) dsts.push_back(1);
         } else {
             dsts = {0, 1, 2, 3};
             if (c.na > 1) angs = {1, 0};
@@ -1786,7 +1789,7 @@ extern "C" int mw3_autotune(mw3_ctx *h, int32_t iterations, int32_t scope, int32
             std::vector<int> xts{c.k_xt}, cws{c.k_cw};
             if (scope & MW3_TUNE_LAYOUT) {
                 if (mw3::xt_eligible(c)) xts = {0, 1};
-                if (c.na > 1 && (c.fp64 || !c.use_tc_ang)) {
+                if (c.na > 1 && !c.use_tc_ang && !c.use_fx_ang) {
                     cws.clear();
                     for (int w = c.ang_cw_fit; w >= 8; w /= 2) cws.push_back(w);
                 }

@@ -1642,6 +1642,9 @@ void launch_hphi(Ctx &c, const double *psi, int g_begin, int g_end)
     } else if (sizeof(T) == 4 && tc_dst_supported(c)) {
         // mixed path: the three DST passes on the tensor cores
         launch_tc_dst(c, (const float *)c.d_X, (float *)c.d_Y, c.d_h, g_begin, g_end, 0);
+    } else if (sizeof(T) == 8 && c.use_fx) {
+        // FP64 path: the four products on the tensor cores
+        launch_fx_dst(c, (const double *)c.d_X, (double *)c.d_Y, c.d_h, g_begin, g_end, true);
     } else {
         // 1. DST along R
         stage_mark(c, 0);
@@ -1680,6 +1683,10 @@ void launch_hphi(Ctx &c, const double *psi, int g_begin, int g_end)
     if (sizeof(T) == 4 && c.use_tc_ang) {
         // mixed path: j^2 + l^2 + Coriolis in one factorised tensor-core contraction
         launch_tc_ang(c, (const float *)c.d_X, c.d_h, g_begin, g_end, c.x_t);
+        stage_mark(c, 4);
+    } else if (sizeof(T) == 8 && c.use_fx_ang) {
+        // FP64 path: the same contraction from exact digits; Y is free after the last transform
+        launch_fx_ang(c, (const double *)c.d_X, (double *)c.d_Y, c.d_h, g_begin, g_end);
         stage_mark(c, 4);
     } else if (c.na > 1) {
         dim3 gj(c.ncj, c.n1, ng);
@@ -2236,26 +2243,36 @@ static void noalloc_hphi(Ctx &c, const WaveTables &t, unsigned char *scratch, co
     int64_t row0 = (int64_t)g0 * na * n1, nrows = (int64_t)ng * na * n1;
     dim3 gr((unsigned)((nrows + BM - 1) / BM), ((n2 + 1) / 2 + BN - 1) / BN);
     const bool rader = sizeof(T) == 8 && c.d_rd_tw;
-    if (rader)
-        k_dst_rows_rader<false><<<rd_grid(), 256, 0, c.stream>>>(d, (const double *)X, (double *)Y, nullptr,
-                                                                 rd_tab(c), g0 * na, ng * na);
-    else
-        k_dst_rows<T, false><<<gr, 256, 0, c.stream>>>(d, X, (const T *)c.d_S2, Y, nullptr, c.d_nopr1, row0, nrows);
-    LAUNCH_CHECK(c);
-    dim3 gc(ng * na, (n2 + COL_W - 1) / COL_W);
-    k_dst_cols<T><<<gc, 256, col_smem(c, sizeof(T)), c.stream>>>(d, Y, (const T *)c.d_S1, c.d_S1off, c.d_nopr1,
-                                                                  c.d_p2r1, c.d_p2r2, c.grid.radcutmax, g0 * na);
-    LAUNCH_CHECK(c);
-    if (rader)
-        k_dst_rows_rader<true><<<rd_grid(), 256, 0, c.stream>>>(d, (const double *)Y, nullptr, H, rd_tab(c), g0 * na,
-                                                                ng * na);
-    else
-        k_dst_rows<T, true><<<gr, 256, 0, c.stream>>>(d, Y, (const T *)c.d_S2, nullptr, H, c.d_nopr1, row0, nrows);
-    LAUNCH_CHECK(c);
+    // the digit products, unless a folded length along r1 needs a second scratch rectangle
+    const bool fx = sizeof(T) == 8 && c.use_fx && !c.d_fxZ;
+    if (fx) {
+        launch_fx_dst(c, (const double *)X, (double *)Y, H, g0, g1, false);
+    } else {
+        if (rader)
+            k_dst_rows_rader<false><<<rd_grid(), 256, 0, c.stream>>>(d, (const double *)X, (double *)Y, nullptr,
+                                                                     rd_tab(c), g0 * na, ng * na);
+        else
+            k_dst_rows<T, false><<<gr, 256, 0, c.stream>>>(d, X, (const T *)c.d_S2, Y, nullptr, c.d_nopr1, row0,
+                                                            nrows);
+        LAUNCH_CHECK(c);
+        dim3 gc(ng * na, (n2 + COL_W - 1) / COL_W);
+        k_dst_cols<T><<<gc, 256, col_smem(c, sizeof(T)), c.stream>>>(d, Y, (const T *)c.d_S1, c.d_S1off, c.d_nopr1,
+                                                                      c.d_p2r1, c.d_p2r2, c.grid.radcutmax, g0 * na);
+        LAUNCH_CHECK(c);
+        if (rader)
+            k_dst_rows_rader<true><<<rd_grid(), 256, 0, c.stream>>>(d, (const double *)Y, nullptr, H, rd_tab(c),
+                                                                    g0 * na, ng * na);
+        else
+            k_dst_rows<T, true><<<gr, 256, 0, c.stream>>>(d, Y, (const T *)c.d_S2, nullptr, H, c.d_nopr1, row0,
+                                                           nrows);
+        LAUNCH_CHECK(c);
+    }
     k_quirk<double><<<ng * na, 128, 0, c.stream>>>(d, P, H, c.d_quirk_ptr, c.d_quirk, g0 * na);
     LAUNCH_CHECK(c);
     if (sizeof(T) == 4 && c.use_tc_ang) {
         launch_tc_ang(c, (const float *)X, H, g0, g1, false);   // its own scratch, [r1][R]
+    } else if (sizeof(T) == 8 && c.use_fx_ang) {
+        launch_fx_ang(c, (const double *)X, (double *)Y, H, g0, g1);
     } else if (na > 1) {
         dim3 gj(c.ncj, n1, ng);
         k_ang_j<T><<<gj, 256, angj_smem(c, sizeof(T)), c.stream>>>(d, X, (const T *)c.d_xj2, H, c.d_tj_ptr, c.d_tj,

@@ -1,0 +1,61 @@
+"""The FP64 path's radial DSTs and angular terms from exact digits on the tensor cores
+against the CPU oracle: even and odd R lengths, lengths along r1 and angles on both sides
+of one 128-row operand, tiles and K steps with remainders, coupled blocks, several
+electronic states, inc = 2, and non-finite input."""
+import os
+
+import numpy as np
+import pytest
+
+from madwave3_gb300 import Propagator
+from oracle.mw3ref import Oracle
+
+pytestmark = pytest.mark.gpu
+
+#        npun1 npun2 nangu  extra
+SHAPES = [(24, 40, 4, {}), (33, 65, 3, {}), (48, 127, 3, {}), (130, 131, 2, {}), (128, 256, 3, {"Jtot": 2, "iommax": 2}),
+          (200, 257, 2, {}), (256, 300, 2, {}), (145, 385, 2, {}), (64, 512, 2, {"nelecmax": 2}),
+          (24, 33, 17, {"Jtot": 4, "iommax": 3}), (28, 40, 64, {"Jtot": 1, "iommax": 1, "iparity": -1}),
+          (24, 36, 129, {}), (20, 34, 145, {"Jtot": 2, "iommax": 2}), (24, 40, 12, {"inc": 2}),
+          (24, 40, 9, {"nelecmax": 3, "lambdas": (0, 1, 0), "Jtot": 2, "iommax": 2})]
+
+
+@pytest.fixture(scope="module")
+def shape_run(tmp_path_factory):
+    from madwave3_gb300.host import generator, setup
+
+    def make(n1, n2, na, extra):
+        d = str(tmp_path_factory.mktemp("fx") / "case")
+        generator.write_case(d, npun1=n1, npun2=n2, nangu=na, jmax=min(na - 1, 12) // 2 * 2, nvmax=1, netot=32, npun1min=8,
+                             alpha0_bohr=1.2, **extra)
+        return setup.load(os.path.join(d, "input.dat"))
+    return make
+
+
+@pytest.mark.parametrize("n1,n2,na,extra", SHAPES)
+def test_hphi_against_the_oracle(shape_run, n1, n2, na, extra):
+    run = shape_run(n1, n2, na, extra)
+    p, ref = Propagator(run, "fp64"), Oracle(run)
+    rng = np.random.default_rng([n1, n2])
+    for psi in (rng.uniform(-1, 1, run.ntot), run.psi0, rng.normal(size=run.ntot) * 10.0 ** rng.uniform(-20, 0, run.ntot)):
+        h, e = p.hphi(psi), ref.hphi(psi)
+        # four products of up to 512 terms and the oracle's own FP64 rounding
+        assert np.abs(h - e).max() <= 1e-13 * np.abs(e).max()
+    assert not p.path()["rader"]
+    p.close()
+
+
+def test_non_finite_input_stays_non_finite(shape_run):
+    run = shape_run(24, 40, 4, {})
+    p = Propagator(run, "fp64")
+    psi = np.random.default_rng(5).uniform(-1, 1, run.ntot)
+    clean = p.hphi(psi)
+    for bad in (np.nan, np.inf, -np.inf):
+        x = psi.copy()
+        x[7] = bad
+        assert not np.isfinite(p.hphi(x)).all()
+    assert np.array_equal(p.hphi(psi), clean)
+    assert np.array_equal(p.hphi(np.zeros(run.ntot)), np.zeros(run.ntot))
+    # subnormal and huge vectors scale as FP64 does
+    assert np.allclose(p.hphi(psi * 2.0 ** 900), clean * 2.0 ** 900, rtol=1e-12)
+    p.close()
