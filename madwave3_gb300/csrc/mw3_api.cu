@@ -1716,7 +1716,7 @@ namespace {
 std::vector<int> path_signature(const Ctx &c)
 {
     const bool explicit_ang = c.na > 1 && !c.use_tc_ang && !c.use_fx_ang;
-    const bool tc3 = !c.fp64 && !c.use_tc_dst2d && mw3::tc_dst_supported(const_cast<Ctx &>(c));
+    const bool tc3 = !c.fp64 && !c.use_tc_dst2d && !c.use_fx && mw3::tc_dst_supported(const_cast<Ctx &>(c));
     return {(int)c.use_tc_dst2d, c.use_tc_dst2d ? (int)c.dst_f16 : -1, (int)tc3, (int)(c.use_tc_ang || c.use_fx_ang), (int)c.x_t,
             (int)(c.fp64 && c.d_rd_tw != nullptr) + 2 * (int)c.use_fx, explicit_ang ? c.ang_cw : 0};
 }
@@ -1765,10 +1765,9 @@ extern "C" int mw3_autotune(mw3_ctx *h, int32_t iterations, int32_t scope, int32
     std::vector<int> dsts{k0[0]}, angs{k0[2]};
     if (scope & MW3_TUNE_FORM) {
         if (c.fp64) {
-            dsts = {-1, 0};              // the digit products, the folded dense ones, Rader where it applies
-            if (c.n2 == 256) dsts.push_back(1);
+            if (c.n2 == 256) dsts = {1, 0, -1};          // -1: the exact-digit products
         } else {
-            dsts = {0, 1, 2, 3};
+            dsts = {0, 1, 2, 3, -1};
             if (c.na > 1) angs = {1, 0};
         }
     }

@@ -1,5 +1,6 @@
-// The radial DST-I products of the FP64 path on the tensor cores (tcgen05.mma,
-// kind::f16) from exact base-256 digits (mw3_fx.cuh).
+// The radial DST-I products and the angular terms on the tensor cores (tcgen05.mma,
+// kind::f16) from exact base-256 digits (mw3_fx.cuh): the FP64 path, and the mixed path's
+// shapes outside its fused chain and its 64-angle kernel.
 //
 // A DST along R or along r1 is y_k = sum_i S[k][i] x_i.  With S[k][n-1-i] = (-1)^k S[k][i]
 // the even outputs come from u_i = x_i + x_{n-1-i} and the odd ones from v_i = x_i -
@@ -20,7 +21,7 @@
 namespace mw3 {
 namespace fx {
 
-// one CTA tile: up to 32 vectors of one segment against one 128-row block of one matrix
+// one CTA tile: up to NV vectors of one segment against one 128-row block of one matrix
 struct alignas(16) Item {
     int seg;
     int v0;          // first vector: r1 row (transforms along R) or column (along r1)
@@ -31,16 +32,17 @@ struct alignas(16) Item {
     int nv;          // vectors
 };
 
+template <typename T>
 struct Args {
     const Item *items;
     int nitems;
     int n1, n2, na;
-    const double *src;
-    double *dst;
+    const T *src;
+    T *dst;
     const unsigned char *planes;
     int pass;                    // 0, 1: the first or the second transform along this axis
     int perm;                    // outputs stored even part first
-    const double *etab;          // along r1, first product: k-space factor [nn][n2], by etoff
+    const T *etab;               // along r1, first product: k-space factor [nn][n2], by etoff
     const int64_t *etoff;        // [W][na]
     int drop;                    // bits the first digit gives up (long sums along R)
     const int *blk_wave;
@@ -50,14 +52,14 @@ struct Args {
     const int64_t *foff;
     // angular terms
     const int *map;
-    const double *yj;            // [G][na][n1] yyy(j, r1) by ladder slot
-    const double *l2;            // [G][3][na][n2] xl2mat_j(Om, Om + q; R), slot q + 1, by ladder slot
+    const T *yj;                 // [G][na][n1] yyy(j, r1) by ladder slot
+    const T *l2;                 // [G][3][na][n2] xl2mat_j(Om, Om + q; R), slot q + 1, by ladder slot
     const int *cpl;              // [G][3][2]: the block Omega + q of the same wave and state, -1 where there is none
     int dexp;                    // the angular matrices' scale 2^dexp
     int *err;
 };
 
-// eight consecutive doubles, zero from n on
+// eight consecutive numbers, zero from n on; vec: they start on 16 bytes
 __device__ __forceinline__ void load8(const double *x, int n, bool vec, double (&v)[8])
 {
     if (vec && n >= 8) {
@@ -70,6 +72,48 @@ __device__ __forceinline__ void load8(const double *x, int n, bool vec, double (
     } else {
 #pragma unroll
         for (int c = 0; c < 8; c++) v[c] = c < n ? x[c] : 0.0;
+    }
+}
+
+__device__ __forceinline__ void load8(const float *x, int n, bool vec, float (&v)[8])
+{
+    if (vec && n >= 8) {
+#pragma unroll
+        for (int c = 0; c < 8; c += 4) {
+            const float4 d = *reinterpret_cast<const float4 *>(x + c);
+            v[c] = d.x;
+            v[c + 1] = d.y;
+            v[c + 2] = d.z;
+            v[c + 3] = d.w;
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < 8; c++) v[c] = c < n ? x[c] : 0.f;
+    }
+}
+
+__device__ __forceinline__ void store8(double *q, int n, bool vec, const double (&y)[8])
+{
+    if (vec && n >= 8) {
+#pragma unroll
+        for (int c = 0; c < 8; c += 2) *reinterpret_cast<double2 *>(q + c) = make_double2(y[c], y[c + 1]);
+    } else {
+#pragma unroll
+        for (int c = 0; c < 8; c++)
+            if (c < n) q[c] = y[c];
+    }
+}
+
+__device__ __forceinline__ void store8(float *q, int n, bool vec, const float (&y)[8])
+{
+    if (vec && n >= 8) {
+#pragma unroll
+        for (int c = 0; c < 8; c += 4)
+            *reinterpret_cast<float4 *>(q + c) = make_float4(y[c], y[c + 1], y[c + 2], y[c + 3]);
+    } else {
+#pragma unroll
+        for (int c = 0; c < 8; c++)
+            if (c < n) q[c] = y[c];
     }
 }
 
@@ -92,14 +136,15 @@ enum Epi { EPI_ROWS = 0, EPI_GATHER = 1, EPI_COLS_E = 2, EPI_COLS = 3, EPI_ANG_J
 
 // eight j-basis values of block g at ladder slot j, r1 row r1 and columns R0..: the j^2 and
 // l^2 terms with the Omega +- 1 blocks, H_b,j = (yyy + l2_0) B_b + l2_- B_{b-1} + l2_+ B_{b+1}
-__device__ __forceinline__ void ang_values(const Args &p, int g, int j, int r1, int R0, int nv, bool vec,
-                                           double (&v)[8])
+template <typename T>
+__device__ __forceinline__ void ang_values(const Args<T> &p, int g, int j, int r1, int R0, int nv, bool vec,
+                                           T (&v)[8])
 {
     const size_t at = ((size_t)j * p.n1 + r1) * p.n2 + R0, blk = (size_t)p.na * p.n1 * p.n2;
-    const double *l = p.l2 + ((size_t)g * 3 * p.na + j) * p.n2 + R0;
+    const T *l = p.l2 + ((size_t)g * 3 * p.na + j) * p.n2 + R0;
     const size_t slot = (size_t)p.na * p.n2;
-    const double y = p.yj[((size_t)g * p.na + j) * p.n1 + r1];
-    double b[8];
+    const T y = p.yj[((size_t)g * p.na + j) * p.n1 + r1];
+    T b[8];
     load8(p.src + g * blk + at, nv, vec, b);
     load8(l + slot, nv, vec, v);
 #pragma unroll
@@ -108,7 +153,7 @@ __device__ __forceinline__ void ang_values(const Args &p, int g, int j, int r1, 
     for (int q = 0; q < 3; q += 2) {
         const int s = p.cpl[(g * 3 + q) * 2];
         if (s < 0) continue;
-        double f[8];
+        T f[8];
         load8(p.src + s * blk + at, nv, vec, b);
         load8(l + q * slot, nv, vec, f);
 #pragma unroll
@@ -116,9 +161,14 @@ __device__ __forceinline__ void ang_values(const Args &p, int g, int j, int r1, 
     }
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(WORKERS, 2) k_fx_dst(Args p)
+template <typename T, int EPI>
+__global__ void __launch_bounds__(WORKERS, 2) k_fx_dst(Args<T> p)
 {
+    typedef typename Num<T>::Int Int;
+    constexpr int ND = Num<T>::ND, NV = Num<T>::NV;
+    constexpr uint32_t ASTEP = Size<T>::ASTEP, BSTEP = Size<T>::BSTEP, BBYTES = Size<T>::BBYTES;
+    // eight vectors a warp; the WPG warps of a group of eight share its K
+    constexpr int NG = NV / 8, WPG = 8 / NG, KT = 32 * WPG, U = KB / KT;
     constexpr bool ROWS = EPI == EPI_ROWS || EPI == EPI_GATHER, ANG = EPI == EPI_ANG_J || EPI == EPI_ANG_G;
     extern __shared__ __align__(128) unsigned char sm[];
     unsigned char *Bs = sm, *As = sm + BBYTES;
@@ -126,7 +176,7 @@ __global__ void __launch_bounds__(WORKERS, 2) k_fx_dst(Args p)
     uint64_t *empty = full + 2, *done = full + 4;
     uint32_t *slot = reinterpret_cast<uint32_t *>(full + 5);
     volatile int *fail = reinterpret_cast<volatile int *>(slot + 1);
-    unsigned *s_max = reinterpret_cast<unsigned *>(slot + 2);      // [2 buffers][2 halves][NV]
+    unsigned *s_max = reinterpret_cast<unsigned *>(slot + 2);      // [2 buffers][WPG][NV]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp == 0) tc::tmem_alloc(slot, 256);
     if (threadIdx.x == 0) {
@@ -169,21 +219,22 @@ __global__ void __launch_bounds__(WORKERS, 2) k_fx_dst(Args p)
     }
     const uint64_t a0 = tc::sdesc(tc::smem_u32(As), LBO, SBO), b0 = tc::sdesc(tc::smem_u32(Bs), LBO, SBO);
     {
-        const int q4 = warp & 3, hf = warp >> 2;
+        const int q4 = warp & 3;
         const int m = q4 * 32 + lane;
         const uint32_t trow = tb + ((uint32_t)(q4 * 32) << 16);
-        const bool vec = (n2 & 1) == 0;           // rows start on 16 bytes
+        const int grp = warp % NG, hf = warp / NG;
+        const bool vec = n2 % (16 / (int)sizeof(T)) == 0;     // rows start on 16 bytes
         int nd = 0, ni = 0;                       // B blocks written, items done
         bool bad = false;
-        double kept[2][8];
+        T kept[U][8];
         // entry k of this thread's eight vectors
-        auto column = [&](const Item &it, int k, double (&v)[8]) {
+        auto column = [&](const Item &it, int k, T (&v)[8]) {
             if (EPI == EPI_ANG_G)
-                ang_values(p, it.seg, k, it.nn, it.v0 + 8 * q4, it.nv - 8 * q4, vec, v);
+                ang_values(p, it.seg, k, it.nn, it.v0 + 8 * grp, it.nv - 8 * grp, vec, v);
             else if (EPI == EPI_ANG_J)
-                load8(p.src + (((size_t)it.seg * p.na + k) * n1 + it.nn) * n2 + it.v0 + 8 * q4, it.nv - 8 * q4, vec, v);
+                load8(p.src + (((size_t)it.seg * p.na + k) * n1 + it.nn) * n2 + it.v0 + 8 * grp, it.nv - 8 * grp, vec, v);
             else
-                load8(p.src + ((size_t)it.seg * n1 + k) * n2 + it.v0 + 8 * q4, it.nv - 8 * q4, vec, v);
+                load8(p.src + ((size_t)it.seg * n1 + k) * n2 + it.v0 + 8 * grp, it.nv - 8 * grp, vec, v);
         };
         for (int i = blockIdx.x; i < p.nitems; i += gridDim.x, ni++) {
             const Item it = p.items[i];
@@ -192,19 +243,23 @@ __global__ void __launch_bounds__(WORKERS, 2) k_fx_dst(Args p)
             const int L = ANG ? p.na : ROWS ? n2 : it.nn;
             const int K = md ? (L + 1) >> 1 : L;
             const int nv = it.nv;
-            const int sh = (md ? 3 : 4) - p.drop;
-            unsigned *sx = s_max + (ni & 1) * 2 * NV;
+            const int sh = Num<T>::SH - (md ? 1 : 0) - p.drop;
+            // the exponent field of vector n's largest |x|
+            auto field = [&](const unsigned *sx, int n) {
+                return (int)((WPG == 2 ? max(sx[n], sx[NV + n]) : sx[n]) >> Num<T>::EBITS);
+            };
+            unsigned *sx = s_max + (ni & 1) * WPG * NV;
             // ---- the largest |x| of each vector ----
             if (ROWS) {
-                const int n = (lane & 7) + 8 * q4, part = (lane >> 3) + 4 * hf;
-                const double *x = p.src + ((size_t)it.seg * n1 + it.v0 + n) * n2;
+                const int n = (lane & 7) + 8 * grp, part = (lane >> 3) + 4 * hf;
+                const T *x = p.src + ((size_t)it.seg * n1 + it.v0 + n) * n2;
                 unsigned mx = 0;
                 if (n < nv)
-                    for (int k = 8 * part; k < L; k += 64) {
-                        double v[8];
+                    for (int k = 8 * part; k < L; k += 8 * 4 * WPG) {
+                        T v[8];
                         load8(x + k, L - k, vec, v);
 #pragma unroll
-                        for (int c = 0; c < 8; c++) mx = max(mx, hi_abs(v[c]));
+                        for (int c = 0; c < 8; c++) mx = max(mx, mag(v[c]));
                     }
                 mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
                 mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
@@ -213,26 +268,28 @@ __global__ void __launch_bounds__(WORKERS, 2) k_fx_dst(Args p)
                 unsigned mx[8];
 #pragma unroll
                 for (int c = 0; c < 8; c++) mx[c] = 0;
-                for (int k = lane + 32 * hf; k < L; k += 64) {
-                    double v[8];
+                // the first B block's entries stay in registers for their digits
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int k = lane + 32 * hf + KT * u;
+                    if (k < L) {
+                        column(it, k, kept[u]);
+#pragma unroll
+                        for (int c = 0; c < 8; c++) mx[c] = max(mx[c], mag(kept[u][c]));
+                    }
+                }
+#pragma unroll 1
+                for (int k = lane + 32 * hf + KB; k < L; k += KT) {
+                    T v[8];
                     column(it, k, v);
 #pragma unroll
-                    for (int c = 0; c < 8; c++) mx[c] = max(mx[c], hi_abs(v[c]));
-                    // a length up to one B block stays in registers for the digits
-                    if (k < KB) {
-                        const int u = k >= 64;
-#pragma unroll
-                        for (int c = 0; c < 8; c++) {
-                            if (u) kept[1][c] = v[c];
-                            else kept[0][c] = v[c];
-                        }
-                    }
+                    for (int c = 0; c < 8; c++) mx[c] = max(mx[c], mag(v[c]));
                 }
                 __syncwarp();
 #pragma unroll
                 for (int c = 0; c < 8; c++) {
                     const unsigned r = __reduce_max_sync(0xffffffffu, mx[c]);
-                    if (lane == c) sx[hf * NV + 8 * q4 + c] = r;
+                    if (lane == c) sx[hf * NV + 8 * grp + c] = r;
                 }
             }
             tc::fence_before_sync();
@@ -241,31 +298,31 @@ __global__ void __launch_bounds__(WORKERS, 2) k_fx_dst(Args p)
             for (int kb = 0; kb < K; kb += KB) {
                 const int kr = (min(K - kb, KB) + KS - 1) & ~(KS - 1);
                 if (ROWS) {
-                    const int n = (lane & 7) + 8 * q4;
-                    const int ef = (int)(max(sx[n], sx[NV + n]) >> 20);
-                    const double *x = p.src + ((size_t)it.seg * n1 + it.v0 + n) * n2;
+                    const int n = (lane & 7) + 8 * grp;
+                    const int ef = field(sx, n);
+                    const T *x = p.src + ((size_t)it.seg * n1 + it.v0 + n) * n2;
 #pragma unroll 1
-                    for (int u = 0; u < 2; u++) {
-                        const int kg = (lane >> 3) + 4 * hf + 8 * u, k = kb + 8 * kg;
+                    for (int u = 0; u < U; u++) {
+                        const int kg = (lane >> 3) + 4 * hf + 4 * WPG * u, k = kb + 8 * kg;
                         if (8 * kg >= kr) continue;
-                        long long X[8];
+                        Int X[8];
 #pragma unroll
                         for (int c = 0; c < 8; c++) X[c] = 0;
                         if (n < nv && k < K) {
-                            double v[8], w[8];
+                            T v[8], w[8];
                             load8(x + k, K - k, vec, v);
                             // x[L-1-k-c]: the eight entries that end at L - 1 - k, backwards
                             const int e = L - 8 - k;
-                            if (e >= 0) load8(x + e, 8, vec && (e & 1) == 0, w);
+                            if (e >= 0) load8(x + e, 8, vec && e % (16 / (int)sizeof(T)) == 0, w);
                             else
 #pragma unroll
-                                for (int c = 0; c < 8; c++) w[c] = e + c >= 0 ? x[e + c] : 0.0;
+                                for (int c = 0; c < 8; c++) w[c] = e + c >= 0 ? x[e + c] : (T)0;
 #pragma unroll
                             for (int c = 0; c < 8; c++) {
                                 const int mr = L - 1 - (k + c);
                                 if (k + c >= K) continue;
                                 X[c] = to_fixed(v[c], ef, sh);
-                                const long long Y = mr != k + c ? to_fixed(w[7 - c], ef, sh) : md == 2 ? X[c] : 0;
+                                const Int Y = mr != k + c ? to_fixed(w[7 - c], ef, sh) : md == 2 ? X[c] : 0;
                                 X[c] = md == 1 ? X[c] + Y : X[c] - Y;
                             }
                         }
@@ -276,16 +333,16 @@ __global__ void __launch_bounds__(WORKERS, 2) k_fx_dst(Args p)
                     int ef[8];
 #pragma unroll
                     for (int c = 0; c < 8; c++)
-                        ef[c] = (int)(max(sx[8 * q4 + c], sx[NV + 8 * q4 + c]) >> 20);
+                        ef[c] = field(sx, 8 * grp + c);
 #pragma unroll
-                    for (int u = 0; u < 2; u++) {
-                        const int kl = lane + 32 * hf + 64 * u, k = kb + kl;
+                    for (int u = 0; u < U; u++) {
+                        const int kl = lane + 32 * hf + KT * u, k = kb + kl;
                         if (kl - lane >= kr) continue;
-                        long long X[8];
+                        Int X[8];
 #pragma unroll
                         for (int c = 0; c < 8; c++) X[c] = 0;
                         if (k < K) {
-                            double v[8];
+                            T v[8];
                             if (kb == 0)
 #pragma unroll
                                 for (int c = 0; c < 8; c++) v[c] = kept[u][c];
@@ -299,7 +356,7 @@ __global__ void __launch_bounds__(WORKERS, 2) k_fx_dst(Args p)
                                     column(it, mr, v);
 #pragma unroll
                                     for (int c = 0; c < 8; c++) {
-                                        const long long Y = to_fixed(v[c], ef[c], sh);
+                                        const Int Y = to_fixed(v[c], ef[c], sh);
                                         X[c] = md == 1 ? X[c] + Y : X[c] - Y;
                                     }
                                 } else if (md == 2) {
@@ -308,7 +365,7 @@ __global__ void __launch_bounds__(WORKERS, 2) k_fx_dst(Args p)
                                 }
                             }
                         }
-                        put_digits(X, Bs + (kl >> 4) * BSTEP + q4 * SBO + ((kl >> 3) & 1) * LBO + (kl & 7) * 16,
+                        put_digits(X, Bs + (kl >> 4) * BSTEP + grp * SBO + ((kl >> 3) & 1) * LBO + (kl & 7) * 16,
                                    NV / 8 * SBO);
                     }
                 }
@@ -322,7 +379,7 @@ __global__ void __launch_bounds__(WORKERS, 2) k_fx_dst(Args p)
                         const int s = t & 1;
                         ok = wait(&full[s], (t >> 1) & 1, fail);
                         if (!ok) break;
-                        step(tb, a0 + (uint64_t)(s * (ASTEP >> 4)), b0 + (uint64_t)(ks * (BSTEP >> 4)), ROWS ? 0 : 1,
+                        step<T>(tb, a0 + (uint64_t)(s * (ASTEP >> 4)), b0 + (uint64_t)(ks * (BSTEP >> 4)), ROWS ? 0 : 1,
                              kb + ks > 0);
                         tc::mma_commit(&empty[s]);
                         t++;
@@ -345,24 +402,24 @@ __global__ void __launch_bounds__(WORKERS, 2) k_fx_dst(Args p)
             }
             bad = bad || *fail;
             bad = __any_sync(0xffffffffu, bad);
-            // ---- epilogue: lane = output, 16 vectors a thread ----
+            // ---- epilogue: lane = output, NV / 2 vectors a thread ----
             const int L2 = (L + 1) >> 1;                                // even outputs
             const int out = 128 * mt + m;                               // index within its parity
             const bool on = !bad && (md == 0 ? out < L : out < (md == 1 ? L2 : L - L2));
             const int k = md == 0 ? out : 2 * out + md - 1;             // the output itself
             const int pos = md == 0 ? out : p.perm && !(L & 1) ? out + (md == 1 ? 0 : L2) : k;
 #pragma unroll 1
-            for (int h = 0; h < 2; h++) {
-                const int c0 = 16 * hf + 8 * h;
+            for (int h = 0; h < NV / 16; h++) {
+                const int c0 = (warp >> 2) * (NV / 2) + 8 * h;
                 uint32_t v[ND][8];
-                load_groups(trow + c0, v);
+                load_groups(trow + c0, NV, v);
                 if (on && c0 < nv) {
-                    double y[8];
+                    T y[8];
 #pragma unroll
                     for (int c = 0; c < 8; c++)
-                        y[c] = combine(v, c, (int)(max(sx[c0 + c], sx[NV + c0 + c]) >> 20), sh + (ANG ? p.dexp : 0));
+                        y[c] = combine(v, c, field(sx, c0 + c), sh + (ANG ? p.dexp : 0));
                     if (EPI == EPI_ROWS) {
-                        double *q = p.dst + ((size_t)it.seg * n1 + it.v0 + c0) * n2 + pos;
+                        T *q = p.dst + ((size_t)it.seg * n1 + it.v0 + c0) * n2 + pos;
 #pragma unroll
                         for (int c = 0; c < 8; c++)
                             if (c0 + c < nv) q[(size_t)c * n2] = y[c];
@@ -374,7 +431,7 @@ __global__ void __launch_bounds__(WORKERS, 2) k_fx_dst(Args p)
                         for (int c = 0; c < 8; c++) idx[c] = c0 + c < nv ? mp[c] : -1;
 #pragma unroll
                         for (int c = 0; c < 8; c++)
-                            if (idx[c] >= 0) h0[idx[c]] = y[c];
+                            if (idx[c] >= 0) h0[idx[c]] = (double)y[c];
                     } else if (EPI == EPI_ANG_G) {
                         // one writer per point: adds at L2, no load in the way
                         const int *mp = p.map + ((size_t)out * n1 + it.nn) * n2 + it.v0 + c0;
@@ -384,26 +441,19 @@ __global__ void __launch_bounds__(WORKERS, 2) k_fx_dst(Args p)
                         for (int c = 0; c < 8; c++) idx[c] = c0 + c < nv ? mp[c] : -1;
 #pragma unroll
                         for (int c = 0; c < 8; c++)
-                            if (idx[c] >= 0) atomicAdd(h0 + idx[c], y[c]);
+                            if (idx[c] >= 0) atomicAdd(h0 + idx[c], (double)y[c]);
                     } else {
-                        double *q = EPI == EPI_ANG_J
+                        T *q = EPI == EPI_ANG_J
                                         ? p.dst + (((size_t)it.seg * p.na + out) * n1 + it.nn) * n2 + it.v0 + c0
                                         : p.dst + ((size_t)it.seg * n1 + pos) * n2 + it.v0 + c0;
                         if (EPI == EPI_COLS_E) {
                             const int wa = p.blk_wave[it.seg / p.na] * p.na + a;
-                            double e[8];
+                            T e[8];
                             load8(p.etab + p.etoff[wa] + (size_t)k * n2 + it.v0 + c0, nv - c0, vec, e);
 #pragma unroll
                             for (int c = 0; c < 8; c++) y[c] *= e[c];
                         }
-                        if (vec && c0 + 8 <= nv) {
-#pragma unroll
-                            for (int c = 0; c < 8; c += 2) *reinterpret_cast<double2 *>(q + c) = make_double2(y[c], y[c + 1]);
-                        } else {
-#pragma unroll
-                            for (int c = 0; c < 8; c++)
-                                if (c0 + c < nv) q[c] = y[c];
-                        }
+                        store8(q, nv - c0, vec, y);
                     }
                 }
                 __syncwarp();
@@ -426,53 +476,60 @@ namespace {
 
 // digits of the rows of one constant matrix, columns col(q), as K steps of 128-row planes
 // (canonical K-major), appended to `out`.  Returns the bits a vector's first digit (up to
-// 512) has to give up so that no group g <= 4 of a row can sum past 2^24
-template <typename F>
+// 512, or 64 of FP32) has to give up so that no group g <= 4 of a row can sum past 2^24.
+// value(m, k): the entry x 2^SBITS, an integer of at most 2^(SBITS+1)
+template <typename T, typename F>
 int append_planes(std::vector<__half> &out, int M, int K, F &&value)
 {
+    constexpr int ND = fx::Num<T>::ND;
+    constexpr uint32_t ASTEP = fx::Size<T>::ASTEP;
+    static const std::vector<__half> half_of = [] {
+        std::vector<__half> h(513);
+        for (int d = 0; d <= 512; d++) h[d] = __float2half((float)(d - 256));
+        return h;
+    }();
+    const double first = sizeof(T) == 8 ? 512.0 : 64.0;       // a vector's first digit
     const int nks = (K + fx::KS - 1) / fx::KS, nmt = (M + 127) / 128;
     const size_t base = out.size();
-    out.resize(base + (size_t)nmt * nks * fx::ASTEP / 2, __float2half(0.f));
+    out.resize(base + (size_t)nmt * nks * ASTEP / 2, half_of[256]);
     int drop = 0;
     for (int m = 0; m < M; m++) {
-        double sum[fx::ND] = {};                // of |digit| over k
+        long long sum[ND] = {};                 // of |digit| over k
         for (int k = 0; k < K; k++) {
-            long long v = (long long)rintl(value(m, k) * 18014398509481984.0L);   // 2^54
-            unsigned char *st = reinterpret_cast<unsigned char *>(out.data() + base) +
-                                ((size_t)(m / 128) * nks + k / fx::KS) * fx::ASTEP +
-                                fx::a_off(m % 128, k % fx::KS);
-            for (int d = fx::ND - 1; d >= 0; d--) {
-                long long g = d > 0 ? ((v + 128) & 255) - 128 : v;
+            long long v = value(m, k);
+            __half *st = out.data() + base +
+                         (((size_t)(m / 128) * nks + k / fx::KS) * ASTEP + fx::a_off(m % 128, k % fx::KS)) / 2;
+            for (int d = ND - 1; d >= 0; d--) {
+                const int g = d > 0 ? (int)((v + 128) & 255) - 128 : (int)v;
                 v = (v - g) >> 8;
-                *reinterpret_cast<__half *>(st + (size_t)d * fx::APL) = __float2half((float)g);
-                sum[d] += (double)(g < 0 ? -g : g);
+                st[(size_t)d * (fx::APL / 2)] = half_of[g + 256];
+                sum[d] += g < 0 ? -g : g;
             }
         }
-        double low = 0.0;                       // digits of x: the first up to 512, the others up to 128
-        for (int g = 0; g < 5; g++) {
-            while (drop < 3 && ldexp(512.0, -drop) * sum[g] + 128.0 * low > 16777216.0) drop++;
-            low += sum[g];
+        double low = 0.0;                       // digits of x past the first: up to 128
+        for (int g = 0; g < std::min(5, ND); g++) {
+            while (drop < 3 && ldexp(first, -drop) * (double)sum[g] + 128.0 * low > 16777216.0) drop++;
+            low += (double)sum[g];
         }
     }
     return drop;
 }
 
-// S[i][k] = 2 sin(pi (i+1)(k+1)/(n+1)) in long double
+// S[i][k] = 2 sin(pi (i+1)(k+1)/(n+1)) x 2^SBITS, rounded from long double
+template <typename T>
 struct Sine {
     int n;
-    std::vector<long double> s;
+    std::vector<long long> s;
     explicit Sine(int n_) : n(n_), s((size_t)2 * (n_ + 1))
     {
         const long double pi = 3.141592653589793238462643383279502884L;
-        for (int m = 0; m < 2 * (n + 1); m++) {
-            // reduced to the first quadrant
-            int q = m % (n + 1);
-            q = std::min(q, n + 1 - q);
-            long double v = 2.0L * sinl(pi * (long double)q / (long double)(n + 1));
-            s[m] = m > n + 1 ? -v : v;
+        for (int m = 0; m <= n + 1; m++) {
+            const int q = std::min(m, n + 1 - m);          // the first quadrant
+            s[m] = llrintl(ldexpl(2.0L * sinl(pi * (long double)q / (long double)(n + 1)), fx::Num<T>::SBITS));
+            if (m > 0 && m <= n) s[2 * (n + 1) - m] = -s[m];
         }
     }
-    long double operator()(int i, int k) const { return s[((long long)(i + 1) * (k + 1)) % (2LL * (n + 1))]; }
+    long long operator()(int i, int k) const { return s[(long long)(i + 1) * (k + 1) % (2 * (n + 1))]; }
 };
 
 // resident CTAs of the persistent kernel: two per SM
@@ -500,20 +557,33 @@ int fx_upload(Ctx &c, V **dst, const std::vector<V> &v)
     return MW3_OK;
 }
 
-}  // namespace
-
-// FP64 path: tables of the digit DSTs; leaves c.use_fx false where the shape is outside them
-int build_fx(Ctx &c)
+template <typename T, int EPI>
+void set_smem()
 {
+    cudaFuncSetAttribute(fx::k_fx_dst<T, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fx::Size<T>::SMEM);
+}
+
+template <typename T, int EPI>
+void launch(Ctx &c, const fx::Args<T> &p)
+{
+    fx::k_fx_dst<T, EPI><<<std::min(p.nitems, c.fx_grid), fx::WORKERS, fx::Size<T>::SMEM, c.stream>>>(p);
+    c.launches++;
+}
+
+template <typename T>
+int build_fx_t(Ctx &c)
+{
+    constexpr int NV = fx::Num<T>::NV;
+    constexpr uint32_t ASTEP = fx::Size<T>::ASTEP;
     c.use_fx = false;
     c.d_fxZ = nullptr;
     // K of one product is at most 256: npun2 <= 512 folded, npun1 <= 256 (which mw3_create asks for)
-    if (!c.fp64 || c.k_dst >= 0 || c.n2 > 512 || c.n1 > 256) return MW3_OK;
+    if (c.n2 > 512 || c.n1 > 256) return MW3_OK;
     const int n1 = c.n1, n2 = c.n2, na = c.na, W = (int)c.waves.size();
     int dropR = 0, drop1 = 0;
     // along R: [pass][parity][128-row block][K step]
     {
-        const Sine S(n2);
+        const Sine<T> S(n2);
         const int he = (n2 + 1) / 2, ho = n2 / 2, K = he;
         const bool perm = n2 % 2 == 0;
         for (int pass = 0; pass < 2; pass++) {
@@ -521,10 +591,10 @@ int build_fx(Ctx &c)
             auto col = [&](int q) { return pass && perm ? 2 * q : q; };
             for (int par = 0; par < 2; par++) {
                 const size_t b = pl.size();
-                dropR = std::max(dropR, append_planes(pl, par ? ho : he, K,
+                dropR = std::max(dropR, append_planes<T>(pl, par ? ho : he, K,
                                                       [&](int m, int k) { return S(2 * m + par, col(k)); }));
                 // both parities take the even one's block count
-                const size_t want = (size_t)((he + 127) / 128) * ((K + fx::KS - 1) / fx::KS) * fx::ASTEP / 2;
+                const size_t want = (size_t)((he + 127) / 128) * ((K + fx::KS - 1) / fx::KS) * ASTEP / 2;
                 pl.resize(b + want, __float2half(0.f));
             }
             __half *d = nullptr;
@@ -539,7 +609,7 @@ int build_fx(Ctx &c)
     {
         std::map<int, std::pair<std::pair<int64_t, int64_t>, int64_t>> at;
         std::vector<__half> pl;
-        std::vector<double> et;
+        std::vector<T> et;
         std::vector<int64_t> eoff((size_t)W * na);
         const int he = (n2 + 1) / 2;
         bool fold = false;
@@ -549,18 +619,18 @@ int build_fx(Ctx &c)
                 const int nn = t.nopr1[a];
                 auto f = at.find(nn);
                 if (f == at.end()) {
-                    const Sine S(nn);
+                    const Sine<T> S(nn);
                     std::pair<int64_t, int64_t> o;
                     o.first = o.second = (int64_t)pl.size() * 2;
                     if (nn <= 128) {
-                        drop1 = std::max(drop1, append_planes(pl, nn, nn, [&](int m, int k) { return S(m, k); }));
+                        drop1 = std::max(drop1, append_planes<T>(pl, nn, nn, [&](int m, int k) { return S(m, k); }));
                     } else {
                         fold = true;
                         const int K = (nn + 1) / 2;
                         for (int pass = 0; pass < (nn % 2 ? 1 : 2); pass++) {
                             if (pass) o.second = (int64_t)pl.size() * 2;
                             for (int par = 0; par < 2; par++)
-                                drop1 = std::max(drop1, append_planes(pl, par ? nn / 2 : K, K, [&](int m, int k) {
+                                drop1 = std::max(drop1, append_planes<T>(pl, par ? nn / 2 : K, K, [&](int m, int k) {
                                                      return S(2 * m + par, pass ? 2 * k : k);
                                                  }));
                         }
@@ -573,12 +643,12 @@ int build_fx(Ctx &c)
                             const int R = n2 % 2 ? q : (q < he ? 2 * q : 2 * (q - he) + 1);
                             double ek = t.p2r1[(size_t)a * n1 + m] + t.p2r2[(size_t)a * n2 + R];
                             if (ek > c.grid.radcutmax) ek = c.grid.radcutmax;
-                            et.push_back(ek * divi);
+                            et.push_back((T)(ek * divi));
                         }
                     f = at.emplace(nn, std::make_pair(o, eo)).first;
                 }
-                off1[(size_t)w * na + a] = (int)(f->second.first.first / fx::ASTEP);
-                off2[(size_t)w * na + a] = (int)(f->second.first.second / fx::ASTEP);
+                off1[(size_t)w * na + a] = (int)(f->second.first.first / ASTEP);
+                off2[(size_t)w * na + a] = (int)(f->second.first.second / ASTEP);
                 eoff[(size_t)w * na + a] = f->second.second;
             }
         if (dropR > 1 || drop1 > 0) return MW3_OK;
@@ -587,19 +657,21 @@ int build_fx(Ctx &c)
         __half *d = nullptr;
         if ((rc = fx_upload(c, &d, pl))) return rc;
         c.d_fxr = d;
-        if ((rc = fx_upload(c, &c.d_fxe, et))) return rc;
+        T *de = nullptr;
+        if ((rc = fx_upload(c, &de, et))) return rc;
+        c.d_fxe = de;
         if ((rc = fx_upload(c, &c.d_fxe_off, eoff))) return rc;
         // a folded product reads rows that another tile of it writes: its own output rectangle
         if (fold) {
             void *z = nullptr;
-            const size_t bytes = sizeof(double) * (size_t)c.G * na * n1 * n2;
+            const size_t bytes = sizeof(T) * (size_t)c.G * na * n1 * n2;
             if (cudaMalloc(&z, bytes) != cudaSuccess) {
                 cudaGetLastError();              // no room: the dense transforms need none
                 return MW3_OK;
             }
             c.allocs.push_back(z);
             MW3_CUDA_TRY(cudaMemset(z, 0, bytes));
-            c.d_fxZ = (double *)z;
+            c.d_fxZ = z;
         }
     }
     // the tiles, in segment order; hphi of a part of the blocks takes a range of them
@@ -612,18 +684,18 @@ int build_fx(Ctx &c)
             for (int a = 0; a < na; a++) {
                 const int seg = (c.waves[w].g0 + b) * na + a, nn = c.waves[w].nopr1[a];
                 const int o1 = off1[(size_t)w * na + a], o2 = off2[(size_t)w * na + a];
-                for (int v = 0; v < nn; v += fx::NV)
+                for (int v = 0; v < nn; v += NV)
                     for (int par = 0; par < 2; par++)
                         for (int mt = 0; mt < (par ? nmto : nmt); mt++) {
                             const int at = (par * nmt + mt) * ksR;
                             rows.push_back(fx::Item{seg, v, (par + 1) | (mt << 2), nn, ksR, {at, at},
-                                                    std::min((int)fx::NV, nn - v)});
+                                                    std::min((int)NV, nn - v)});
                         }
                 const int K1 = nn <= 128 ? nn : (nn + 1) / 2, ks1 = (K1 + fx::KS - 1) / fx::KS;
-                for (int v = 0; v < n2; v += fx::NV)
+                for (int v = 0; v < n2; v += NV)
                     for (int par = 0; par < (nn <= 128 ? 1 : 2); par++)
                         cols.push_back(fx::Item{seg, v, nn <= 128 ? 0 : par + 1, nn, ks1,
-                                                {o1 + par * ks1, o2 + par * ks1}, std::min((int)fx::NV, n2 - v)});
+                                                {o1 + par * ks1, o2 + par * ks1}, std::min((int)NV, n2 - v)});
                 c.h_fx_row0.push_back((int)rows.size());
                 c.h_fx_col0.push_back((int)cols.size());
             }
@@ -633,23 +705,24 @@ int build_fx(Ctx &c)
     c.d_fx_rows = d;
     if ((rc = fx_upload(c, &d, cols))) return rc;
     c.d_fx_cols = d;
-    cudaFuncSetAttribute(fx::k_fx_dst<fx::EPI_ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fx::SMEM);
-    cudaFuncSetAttribute(fx::k_fx_dst<fx::EPI_GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fx::SMEM);
-    cudaFuncSetAttribute(fx::k_fx_dst<fx::EPI_COLS_E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fx::SMEM);
-    cudaFuncSetAttribute(fx::k_fx_dst<fx::EPI_COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fx::SMEM);
+    set_smem<T, fx::EPI_ROWS>();
+    set_smem<T, fx::EPI_GATHER>();
+    set_smem<T, fx::EPI_COLS_E>();
+    set_smem<T, fx::EPI_COLS>();
     c.fx_grid = fx_ctas();
     c.use_fx = true;
     return MW3_OK;
 }
 
-// FP64 path: the angular terms through the j basis, B = D X, the j-diagonal scaling with the
+// the angular terms through the j basis, B = D X, the j-diagonal scaling with the
 // Omega +- 1 coupling, H += D^T Hb, both products from exact digits.  Leaves c.use_fx_ang
 // false where the explicit matrices are needed (over 256 angles, a block whose j list leaves
 // the ladder j0 + k inc, or matrices the digits do not cover)
-int build_fx_ang(Ctx &c)
+template <typename T>
+int build_fx_ang_t(Ctx &c)
 {
-    c.use_fx_ang = false;
-    if (!c.fp64 || c.k_ang == 0 || c.na < 2 || c.na > 256) return MW3_OK;
+    constexpr int NV = fx::Num<T>::NV;
+    constexpr uint32_t ASTEP = fx::Size<T>::ASTEP;
     const int na = c.na, n1 = c.n1, n2 = c.n2, G = c.G, ne = c.ne;
     const int nks = (na + fx::KS - 1) / fx::KS, nmt = (na + 127) / 128;
     double dmax = 0.0;
@@ -664,7 +737,7 @@ int build_fx_ang(Ctx &c)
     std::vector<__half> pl;
     std::vector<const double *> seen;                 // the (Omega, state) columns already cut
     std::vector<int> seen_at, seen_lad;
-    std::vector<double> yj((size_t)G * na * n1, 0.0), l2((size_t)G * 3 * na * n2, 0.0);
+    std::vector<T> yj((size_t)G * na * n1, (T)0), l2((size_t)G * 3 * na * n2, (T)0);
     std::vector<int> at((size_t)G * 2);
     int drop = 0;
     for (auto &t : c.waves) {
@@ -685,12 +758,13 @@ int build_fx_ang(Ctx &c)
                 f = (int)seen.size();
                 seen.push_back(D);
                 seen_lad.push_back(lad);
-                seen_at.push_back((int)(pl.size() * 2 / fx::ASTEP));
+                seen_at.push_back((int)(pl.size() * 2 / ASTEP));
                 auto d = [&](int js, int a) {
-                    return js < njl ? ldexpl((long double)D[(size_t)(t.j0 + js * t.inc) * na + a], dexp) : 0.0L;
+                    return js < njl ? llrint(ldexp(D[(size_t)(t.j0 + js * t.inc) * na + a], dexp + fx::Num<T>::SBITS))
+                                    : 0LL;
                 };
-                drop = std::max(drop, append_planes(pl, na, na, [&](int m, int k) { return d(m, k); }));
-                drop = std::max(drop, append_planes(pl, na, na, [&](int m, int k) { return d(k, m); }));
+                drop = std::max(drop, append_planes<T>(pl, na, na, [&](int m, int k) { return d(m, k); }));
+                drop = std::max(drop, append_planes<T>(pl, na, na, [&](int m, int k) { return d(k, m); }));
             }
             at[2 * g] = seen_at[f];
             at[2 * g + 1] = seen_at[f] + nmt * nks;
@@ -703,7 +777,7 @@ int build_fx_ang(Ctx &c)
                 if ((jb - t.j0) % t.inc != 0 || (jb - t.j0) / t.inc < 0 || (jb - t.j0) / t.inc >= njl) return MW3_OK;
                 const int js = (jb - t.j0) / t.inc;
                 for (int ir1 = 0; ir1 < n1; ir1++)
-                    yj[((size_t)g * na + js) * n1 + ir1] += t.yj2[((size_t)b * n1 + ir1) * na + k];
+                    yj[((size_t)g * na + js) * n1 + ir1] += (T)t.yj2[((size_t)b * n1 + ir1) * na + k];
             }
             // xl2mat_j(Om, Om + q; R) for the sources Om + q
             for (int q = -1; q <= 1; q++) {
@@ -714,19 +788,19 @@ int build_fx_ang(Ctx &c)
                     if (!t.l2used[u]) continue;
                     for (int ir2 = 0; ir2 < n2; ir2++)
                         l2[(((size_t)g * 3 + (q + 1)) * na + js) * n2 + ir2] =
-                            t.l2tab[((((size_t)(e - 1) * t.nj2 + js) * n2 + ir2) * t.nom + (om - t.iommin)) * t.nom +
-                                    (oms - t.iommin)];
+                            (T)t.l2tab[((((size_t)(e - 1) * t.nj2 + js) * n2 + ir2) * t.nom + (om - t.iommin)) * t.nom +
+                                       (oms - t.iommin)];
                 }
             }
         }
     }
     if (drop > 1) return MW3_OK;
-    // tiles of one r1 row x 32 R that hold stored points
-    const int t2n = (n2 + fx::NV - 1) / fx::NV;
+    // tiles of one r1 row x NV R that hold stored points
+    const int t2n = (n2 + NV - 1) / NV;
     std::vector<char> on((size_t)n1 * t2n, 0);
     for (int a = 0; a < na; a++)
         for (int ir = 0; ir < c.npunreal[a]; ir++)
-            on[(size_t)(c.indr1[(size_t)a * c.npt + ir] - 1) * t2n + (c.indr2[(size_t)a * c.npt + ir] - 1) / fx::NV] = 1;
+            on[(size_t)(c.indr1[(size_t)a * c.npt + ir] - 1) * t2n + (c.indr2[(size_t)a * c.npt + ir] - 1) / NV] = 1;
     std::vector<fx::Item> items;
     c.h_fx_ang0.assign(1, 0);
     for (int g = 0; g < G; g++) {
@@ -734,8 +808,8 @@ int build_fx_ang(Ctx &c)
             for (int j = 0; j < t2n; j++)
                 if (on[(size_t)i * t2n + j])
                     for (int mt = 0; mt < nmt; mt++)
-                        items.push_back(fx::Item{g, j * fx::NV, mt << 2, i, nks, {at[2 * g] + mt * nks, at[2 * g + 1] + mt * nks},
-                                                 std::min((int)fx::NV, n2 - j * fx::NV)});
+                        items.push_back(fx::Item{g, j * NV, mt << 2, i, nks, {at[2 * g] + mt * nks, at[2 * g + 1] + mt * nks},
+                                                 std::min((int)NV, n2 - j * NV)});
         c.h_fx_ang0.push_back((int)items.size());
     }
     int rc;
@@ -743,75 +817,96 @@ int build_fx_ang(Ctx &c)
     fx::Item *di = nullptr;
     if ((rc = fx_upload(c, &d, pl))) return rc;
     if ((rc = fx_upload(c, &di, items))) return rc;
-    if ((rc = fx_upload(c, &c.d_fx_yj, yj))) return rc;
-    if ((rc = fx_upload(c, &c.d_fx_l2, l2))) return rc;
+    T *dy = nullptr, *dl = nullptr;
+    if ((rc = fx_upload(c, &dy, yj))) return rc;
+    if ((rc = fx_upload(c, &dl, l2))) return rc;
+    c.d_fx_yj = dy;
+    c.d_fx_l2 = dl;
     c.d_fx_ang = di;
     c.d_fxD = d;
     c.fx_drop_ang = drop;
     c.fx_dexp = dexp;
-    cudaFuncSetAttribute(fx::k_fx_dst<fx::EPI_ANG_J>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fx::SMEM);
-    cudaFuncSetAttribute(fx::k_fx_dst<fx::EPI_ANG_G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fx::SMEM);
+    set_smem<T, fx::EPI_ANG_J>();
+    set_smem<T, fx::EPI_ANG_G>();
     c.fx_grid = fx_ctas();
     c.use_fx_ang = true;
     return MW3_OK;
 }
 
-// j^2, l^2 and the Omega coupling of blocks [g_begin, g_end) (whole waves): X -> B in Y, then H +=
-void launch_fx_ang(Ctx &c, const double *X, double *Y, double *H, int g_begin, int g_end)
+}  // namespace
+
+// tables of the digit DSTs; leaves c.use_fx false where another path is asked for or faster
+// (mixed: the fused chain) or the shape is outside them
+int build_fx(Ctx &c)
 {
-    fx::Args p = {};
+    c.use_fx = false;
+    c.d_fxZ = nullptr;
+    if (c.k_dst >= 0 || (!c.fp64 && c.use_tc_dst2d)) return MW3_OK;
+    return c.fp64 ? build_fx_t<double>(c) : build_fx_t<float>(c);
+}
+
+int build_fx_ang(Ctx &c)
+{
+    c.use_fx_ang = false;
+    if (c.k_ang == 0 || c.na < 2 || c.na > 256 || c.use_tc_ang) return MW3_OK;
+    return c.fp64 ? build_fx_ang_t<double>(c) : build_fx_ang_t<float>(c);
+}
+
+// j^2, l^2 and the Omega coupling of blocks [g_begin, g_end) (whole waves): X -> B in Y, then H +=
+template <typename T>
+void launch_fx_ang(Ctx &c, const T *X, T *Y, double *H, int g_begin, int g_end)
+{
+    fx::Args<T> p = {};
     p.n1 = c.n1; p.n2 = c.n2; p.na = c.na;
     p.blk_wave = c.d_blk_wave;
     p.H = H; p.map = c.d_map; p.foff = c.d_foff;
     p.err = c.d_tc_err;
     p.planes = (const unsigned char *)c.d_fxD;
-    p.yj = c.d_fx_yj; p.l2 = c.d_fx_l2; p.cpl = c.d_cpl;
+    p.yj = (const T *)c.d_fx_yj; p.l2 = (const T *)c.d_fx_l2; p.cpl = c.d_cpl;
     p.drop = c.fx_drop_ang; p.dexp = c.fx_dexp;
     p.items = (const fx::Item *)c.d_fx_ang + c.h_fx_ang0[g_begin];
     p.nitems = c.h_fx_ang0[g_end] - c.h_fx_ang0[g_begin];
-    const int grid = std::min(p.nitems, c.fx_grid);
     p.src = X; p.dst = Y; p.pass = 0;
-    fx::k_fx_dst<fx::EPI_ANG_J><<<grid, fx::WORKERS, fx::SMEM, c.stream>>>(p);
-    c.launches++;
+    launch<T, fx::EPI_ANG_J>(c, p);
     p.src = Y; p.dst = nullptr; p.pass = 1;
-    fx::k_fx_dst<fx::EPI_ANG_G><<<grid, fx::WORKERS, fx::SMEM, c.stream>>>(p);
-    c.launches++;
+    launch<T, fx::EPI_ANG_G>(c, p);
 }
 
 // the four products of the radial kinetic term of blocks [g_begin, g_end): X -> Y, Y in place
 // (or through Z), Y -> H at the stored points
-void launch_fx_dst(Ctx &c, const double *X, double *Y, double *H, int g_begin, int g_end, bool mark)
+template <typename T>
+void launch_fx_dst(Ctx &c, const T *X, T *Y, double *H, int g_begin, int g_end, bool mark)
 {
     const int s0 = g_begin * c.na, s1 = g_end * c.na;
-    fx::Args p = {};
+    fx::Args<T> p = {};
     p.n1 = c.n1; p.n2 = c.n2; p.na = c.na;
     p.blk_wave = c.d_blk_wave;
     p.H = H; p.mapT = c.d_mapT; p.foff = c.d_foff;
     p.err = c.d_tc_err;
-    p.etab = c.d_fxe; p.etoff = c.d_fxe_off;
+    p.etab = (const T *)c.d_fxe; p.etoff = c.d_fxe_off;
     const fx::Item *rows = (const fx::Item *)c.d_fx_rows + c.h_fx_row0[s0];
     const fx::Item *cols = (const fx::Item *)c.d_fx_cols + c.h_fx_col0[s0];
     const int nr = c.h_fx_row0[s1] - c.h_fx_row0[s0], nc = c.h_fx_col0[s1] - c.h_fx_col0[s0];
-    const int gr = std::min(nr, c.fx_grid), gc = std::min(nc, c.fx_grid);
     if (mark) stage_mark(c, 0);
     p.items = rows; p.nitems = nr;
     p.src = X; p.dst = Y; p.planes = (const unsigned char *)c.d_fxR[0]; p.perm = 1; p.pass = 0; p.drop = c.fx_drop;
-    fx::k_fx_dst<fx::EPI_ROWS><<<gr, fx::WORKERS, fx::SMEM, c.stream>>>(p);
-    c.launches++;
+    launch<T, fx::EPI_ROWS>(c, p);
     if (mark) stage_mark(c, 1);
-    double *Z = c.d_fxZ ? c.d_fxZ : Y;
+    T *Z = c.d_fxZ ? (T *)c.d_fxZ : Y;
     p.items = cols; p.nitems = nc;
     p.src = Y; p.dst = Z; p.planes = (const unsigned char *)c.d_fxr; p.drop = 0;
-    fx::k_fx_dst<fx::EPI_COLS_E><<<gc, fx::WORKERS, fx::SMEM, c.stream>>>(p);
-    c.launches++;
+    launch<T, fx::EPI_COLS_E>(c, p);
     p.src = Z; p.dst = Y; p.perm = 0; p.pass = 1;
-    fx::k_fx_dst<fx::EPI_COLS><<<gc, fx::WORKERS, fx::SMEM, c.stream>>>(p);
-    c.launches++;
+    launch<T, fx::EPI_COLS>(c, p);
     if (mark) stage_mark(c, 2);
     p.items = rows; p.nitems = nr;
     p.src = Y; p.dst = nullptr; p.planes = (const unsigned char *)c.d_fxR[1]; p.drop = c.fx_drop;
-    fx::k_fx_dst<fx::EPI_GATHER><<<gr, fx::WORKERS, fx::SMEM, c.stream>>>(p);
-    c.launches++;
+    launch<T, fx::EPI_GATHER>(c, p);
 }
+
+template void launch_fx_dst<double>(Ctx &, const double *, double *, double *, int, int, bool);
+template void launch_fx_dst<float>(Ctx &, const float *, float *, double *, int, int, bool);
+template void launch_fx_ang<double>(Ctx &, const double *, double *, double *, int, int);
+template void launch_fx_ang<float>(Ctx &, const float *, float *, double *, int, int);
 
 }  // namespace mw3

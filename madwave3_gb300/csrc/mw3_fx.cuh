@@ -7,9 +7,9 @@
 // groups past 6 that are left out are 2^-54 of a typical row sum, below one FP64 rounding.  (Error-free splitting
 // of matrix products after Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59, 2012.)
 //
-// All digits of one K step of B stand one below the other (row = 32 digit + vector), so
-// digit i of A takes the first 7 - i digits of B in one MMA of N = 32 (7 - i) whose
-// columns start at 32 i: group g = i + j lands in columns 32 g .. 32 g + 31 by itself.
+// All digits of one K step of B stand one below the other (row = NV digit + vector), so
+// digit i of A takes the first ND - i digits of B in one MMA of N = NV (ND - i) whose
+// columns start at NV i: group g = i + j lands in columns NV g .. NV g + NV - 1 by itself.
 #pragma once
 #include "mw3_tc.cuh"
 
@@ -18,18 +18,30 @@
 namespace mw3 {
 namespace fx {
 
-constexpr int ND = 7;                              // digits
-constexpr int NV = 32;                             // vectors of one tile
 constexpr int KS = 16;                             // K of one MMA
 constexpr int KB = 128;                            // K of one B block in shared memory
 constexpr uint32_t APL = 128 * KS * 2;             // one digit of one K step of A: 4 KB
-constexpr uint32_t ASTEP = ND * APL;               // 28 KB
-constexpr uint32_t BSTEP = ND * NV * KS * 2;       // 7 KB
-constexpr uint32_t BBYTES = (KB / KS) * BSTEP;     // 56 KB
 constexpr uint32_t SBO = 256, LBO = 128;
 constexpr int WORKERS = 256;
-constexpr uint32_t SMALL = 1024;
-constexpr uint32_t SMEM = BBYTES + 2 * ASTEP + SMALL;   // 113 KB: two CTAs per SM
+
+// What depends on the type of the vectors.  FP32 vectors take four digits of 30 bits
+// (|X| <= 2^30, the constant matrix x 2^29), FP64 vectors seven; the accumulators of all
+// groups of one tile fill up to 256 tensor-memory columns, so two CTAs share an SM.
+template <typename T> struct Num;
+template <> struct Num<double> {
+    enum { ND = 7, NV = 32, SH = 4, EBITS = 20, EMAX = 0x7FF, SBITS = 54 };
+    typedef long long Int;
+};
+template <> struct Num<float> {
+    enum { ND = 4, NV = 64, SH = 6, EBITS = 23, EMAX = 0xFF, SBITS = 29 };
+    typedef int Int;
+};
+template <typename T> struct Size {
+    static constexpr uint32_t ASTEP = Num<T>::ND * APL;                            // 28 or 16 KB
+    static constexpr uint32_t BSTEP = Num<T>::ND * Num<T>::NV * KS * 2;            // 7 or 8 KB
+    static constexpr uint32_t BBYTES = (KB / KS) * BSTEP;                          // 56 or 64 KB
+    static constexpr uint32_t SMEM = BBYTES + 2 * ASTEP + 1024;                    // 113 or 97 KB
+};
 
 // element (row, k) of one digit of a K step of A
 __host__ __device__ constexpr uint32_t a_off(int r, int k)
@@ -37,7 +49,9 @@ __host__ __device__ constexpr uint32_t a_off(int r, int k)
     return (uint32_t)((r & 7) * 16 + (r >> 3) * SBO + (k & 7) * 2 + (k >> 3) * LBO);
 }
 
-__device__ __forceinline__ unsigned hi_abs(double x) { return (unsigned)__double2hiint(x) & 0x7FFFFFFFu; }
+// the bits of |x| that order vectors' entries: the high word, or all of an FP32 number
+__device__ __forceinline__ unsigned mag(double x) { return (unsigned)__double2hiint(x) & 0x7FFFFFFFu; }
+__device__ __forceinline__ unsigned mag(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }
 
 // round(x 2^(57 - E)) for |x| < 2^E, E = ef - 1022 with ef the exponent field of the
 // largest |x| of the vector; sh = 4, or 3 to leave a bit for a sum of two
@@ -53,6 +67,24 @@ __device__ __forceinline__ long long to_fixed(double x, int ef, int sh)
     return ((long long)v ^ s) - s;
 }
 
+// the same in 32 bits: round(x 2^(30 - E)), E = ef - 126, for sh = 6
+__device__ __forceinline__ int to_fixed(float x, int ef, int sh)
+{
+    const unsigned b = __float_as_uint(x);
+    const int ex = (int)((b >> 23) & 0xFFu);
+    const unsigned r = min((unsigned)(ef - max(ex, 1)), 31u);
+    unsigned v = ((b & 0x7FFFFFu) | (ex ? 0x800000u : 0u)) << sh;
+    v = (v + ((1u << r) >> 1)) >> r;
+    const int s = (int)b >> 31;
+    return ((int)v ^ s) - s;
+}
+
+__device__ __forceinline__ uint32_t h2sub(uint32_t u, __half2 off)
+{
+    const __half2 v = __hsub2(*reinterpret_cast<const __half2 *>(&u), off);
+    return *reinterpret_cast<const uint32_t *>(&v);
+}
+
 // the seven digits of eight integers (|X| <= 2^57) as FP16, 16 bytes a digit
 __device__ __forceinline__ void put_digits(const long long *X, unsigned char *dst, uint32_t digit_stride)
 {
@@ -66,7 +98,7 @@ __device__ __forceinline__ void put_digits(const long long *X, unsigned char *ds
     // 1024 of the bit pattern and the bias, 512 or 128
     const __half2 off0 = __floats2half2_rn(1536.f, 1536.f), off = __floats2half2_rn(1152.f, 1152.f);
 #pragma unroll
-    for (int d = 0; d < ND; d++) {
+    for (int d = 0; d < 7; d++) {
         uint32_t w[4];
 #pragma unroll
         for (int p = 0; p < 4; p++) {
@@ -79,20 +111,39 @@ __device__ __forceinline__ void put_digits(const long long *X, unsigned char *ds
                 u = (__byte_perm(lo[2 * p], lo[2 * p + 1], (unsigned)(by | ((4 + by) << 8))) & 0x00FF00FFu) |
                     0x64006400u;
             }
-            const __half2 v = __hsub2(*reinterpret_cast<const __half2 *>(&u), d ? off : off0);
-            w[p] = *reinterpret_cast<const uint32_t *>(&v);
+            w[p] = h2sub(u, d ? off : off0);
         }
         *reinterpret_cast<uint4 *>(dst + d * digit_stride) = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
-// one accumulator row of eight vectors: v[g][c], g the group; the sum over k S x in FP64.
-// ef: exponent field of the vector's largest |x|, sh as in to_fixed
-__device__ __forceinline__ double combine(const uint32_t (&v)[ND][8], int c, int ef, int sh)
+// the four digits of eight integers (|X| <= 2^30)
+__device__ __forceinline__ void put_digits(const int *X, unsigned char *dst, uint32_t digit_stride)
 {
-    int a[ND];
+    uint32_t b[8];
 #pragma unroll
-    for (int g = 0; g < ND; g++) a[g] = __float2int_rn(__uint_as_float(v[g][c]));
+    for (int i = 0; i < 8; i++) b[i] = (uint32_t)X[i] + 0x80808080u;
+    const __half2 off = __floats2half2_rn(1152.f, 1152.f);
+#pragma unroll
+    for (int d = 0; d < 4; d++) {
+        const int by = 3 - d;
+        uint32_t w[4];
+#pragma unroll
+        for (int p = 0; p < 4; p++)
+            w[p] = h2sub((__byte_perm(b[2 * p], b[2 * p + 1], (unsigned)(by | ((4 + by) << 8))) & 0x00FF00FFu) |
+                             0x64006400u,
+                         off);
+        *reinterpret_cast<uint4 *>(dst + d * digit_stride) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+// one accumulator row of eight vectors: v[g][c], g the group; the sum over k of S x.
+// ef: exponent field of the vector's largest |x|, sh as in to_fixed
+__device__ __forceinline__ double combine(const uint32_t (&v)[7][8], int c, int ef, int sh)
+{
+    int a[7];
+#pragma unroll
+    for (int g = 0; g < 7; g++) a[g] = __float2int_rn(__uint_as_float(v[g][c]));
     const long long H = ((long long)a[0] << 24) + ((long long)a[1] << 16) + ((long long)a[2] << 8) + a[3];
     const long long L = ((long long)a[4] << 16) + ((long long)a[5] << 8) + a[6];
     // the leading 62 bits of H 2^24 + L, in units 2^(72-z) of 2^54 2^(57-E)
@@ -106,6 +157,20 @@ __device__ __forceinline__ double combine(const uint32_t (&v)[ND][8], int c, int
     if (e > 0 && e < 0x7FF)
         return __hiloint2double(__double2hiint(y) + (sc << 20), __double2loint(y));
     return scalbn(y, sc);
+}
+
+// the groups are exact; their FP32 sum rounds once at the size of the first
+__device__ __forceinline__ float combine(const uint32_t (&v)[4][8], int c, int ef, int sh)
+{
+    const float r = 1.f / 256.f;
+    const float f = fmaf(fmaf(fmaf(__uint_as_float(v[3][c]), r, __uint_as_float(v[2][c])), r, __uint_as_float(v[1][c])),
+                         r, __uint_as_float(v[0][c]));
+    if (ef >= 0xFF) return __uint_as_float(0x7FC00000u);
+    const int sc = ef - 137 + (6 - sh);              // E - 11 (48 - 29 - 30), one more for a folded vector
+    const int s0 = max(sc, -100);
+    float y = f * __uint_as_float((unsigned)(s0 + 127) << 23);
+    if (sc < -100) y *= __uint_as_float((unsigned)(sc + 227) << 23);
+    return y;
 }
 
 __device__ __forceinline__ bool wait(uint64_t *mbar, uint32_t parity, volatile int *fail)
@@ -134,11 +199,6 @@ __device__ __forceinline__ bool wait(uint64_t *mbar, uint32_t parity, volatile i
     }
 }
 
-__device__ __forceinline__ void arrive(uint64_t *mbar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" : : "r"(tc::smem_u32(mbar)) : "memory");
-}
-
 __device__ __forceinline__ void mma_f16(uint32_t dtmem, uint64_t ad, uint64_t bd, uint32_t idesc, int accumulate)
 {
     asm volatile(
@@ -156,8 +216,10 @@ __host__ __device__ constexpr uint32_t idesc(int M, int N, int bmn)
 }
 
 // the MMAs of one K step: A at a (ND planes), B at b
+template <typename T>
 __device__ __forceinline__ void step(uint32_t d, uint64_t a, uint64_t b, int bmn, int accumulate)
 {
+    constexpr int ND = Num<T>::ND, NV = Num<T>::NV;
 #pragma unroll
     for (int i = 0; i < ND; i++)
         mma_f16(d + NV * i, a + (uint64_t)(i * (APL >> 4)), b, idesc(128, NV * (ND - i), bmn), i ? 1 : accumulate);
@@ -176,11 +238,12 @@ __device__ __forceinline__ void regs8(uint32_t *r)
     asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]));
 }
 
-// the ND accumulators of eight columns of this thread's lane
-__device__ __forceinline__ void load_groups(uint32_t taddr, uint32_t (&v)[ND][8])
+// the accumulators of eight columns of this thread's lane, groups nv columns apart
+template <int ND>
+__device__ __forceinline__ void load_groups(uint32_t taddr, int nv, uint32_t (&v)[ND][8])
 {
 #pragma unroll
-    for (int g = 0; g < ND; g++) ld8_nw(taddr + NV * g, v[g]);
+    for (int g = 0; g < ND; g++) ld8_nw(taddr + nv * g, v[g]);
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int g = 0; g < ND; g++) regs8(v[g]);

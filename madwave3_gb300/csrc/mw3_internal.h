@@ -201,21 +201,21 @@ struct Ctx {
     int *d_rd_out = nullptr;         // p -> output column | (odd output) << 16
     int64_t *d_rowpre = nullptr;     // [G na + 1]: rows ir1 < nopr1 before each segment
     int64_t *d_S1off = nullptr;      // [W][na]
-    // FP64 path: the DSTs from exact digits on the tensor cores (mw3_fx.cu)
+    // the DSTs from exact digits on the tensor cores (mw3_fx.cu): FP64, and mixed shapes outside the fused chain
     bool use_fx = false;
     int fx_grid = 0, fx_drop = 0;
     void *d_fxR[2] = {nullptr, nullptr};   // digits of S2: first and second transform (__half planes)
     void *d_fxr = nullptr;           // digits of S1 of every length
-    double *d_fxe = nullptr;         // k-space factor of every length, [nn][n2] by stored column
+    void *d_fxe = nullptr;           // k-space factor of every length, [nn][n2] by stored column
     int64_t *d_fxe_off = nullptr;    // [W][na]
-    double *d_fxZ = nullptr;         // second scratch rectangle, where a length exceeds 128
+    void *d_fxZ = nullptr;           // second scratch rectangle, where a length exceeds 128
     void *d_fx_rows = nullptr, *d_fx_cols = nullptr;     // the tiles
     std::vector<int> h_fx_row0, h_fx_col0;               // [G na + 1] first tile of each segment
-    // FP64 path: the angular terms through the j basis, from exact digits
+    // the angular terms through the j basis, from exact digits: FP64, and mixed above 64 angles
     bool use_fx_ang = false;
     int fx_drop_ang = 0, fx_dexp = 0;
     void *d_fxD = nullptr;           // digits of Djmmp, both directions, per distinct (Omega, state)
-    double *d_fx_yj = nullptr, *d_fx_l2 = nullptr;       // [G][na][n1], [G][3][na][n2] by ladder slot
+    void *d_fx_yj = nullptr, *d_fx_l2 = nullptr;         // [G][na][n1], [G][3][na][n2] by ladder slot
     void *d_fx_ang = nullptr;        // the tiles
     std::vector<int> h_fx_ang0;                          // [G + 1] first tile of each block
     // explicit angular kinetic matrices (type T)
@@ -398,12 +398,14 @@ int encode_tc_dst2d_xmap(Ctx &c);
 bool xt_eligible(const Ctx &c);
 void launch_tc_dst2d(Ctx &c, const float *X, float *H, int g_begin, int g_end);
 std::vector<double> dst_matrix(int n);
-// FP64 radial DSTs from exact digits (mw3_fx.cu); sets c.use_fx
+// radial DSTs from exact digits (mw3_fx.cu); sets c.use_fx
 int build_fx(Ctx &c);
-void launch_fx_dst(Ctx &c, const double *X, double *Y, double *H, int g_begin, int g_end, bool mark);
-// FP64 angular terms through the j basis; sets c.use_fx_ang
+template <typename T>
+void launch_fx_dst(Ctx &c, const T *X, T *Y, double *H, int g_begin, int g_end, bool mark);
+// angular terms through the j basis, from exact digits; sets c.use_fx_ang
 int build_fx_ang(Ctx &c);
-void launch_fx_ang(Ctx &c, const double *X, double *Y, double *H, int g_begin, int g_end);
+template <typename T>
+void launch_fx_ang(Ctx &c, const T *X, T *Y, double *H, int g_begin, int g_end);
 
 // ---------------------------------------------------------------------------
 // setup (mw3_setup.cu)

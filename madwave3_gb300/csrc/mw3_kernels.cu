@@ -1639,12 +1639,12 @@ void launch_hphi(Ctx &c, const double *psi, int g_begin, int g_end)
         // the explicit angular kernels accumulate in FP64: widen H first
         k_h32_to_h<<<dim3(ng * c.na, c.nchunk), 256, 0, c.stream>>>(d, c.d_h32, c.d_h, g_begin * c.na);
         LAUNCH_CHECK(c);
+    } else if (c.use_fx) {
+        // the four products from exact digits on the tensor cores
+        launch_fx_dst<T>(c, (const T *)c.d_X, (T *)c.d_Y, c.d_h, g_begin, g_end, true);
     } else if (sizeof(T) == 4 && tc_dst_supported(c)) {
         // mixed path: the three DST passes on the tensor cores
         launch_tc_dst(c, (const float *)c.d_X, (float *)c.d_Y, c.d_h, g_begin, g_end, 0);
-    } else if (sizeof(T) == 8 && c.use_fx) {
-        // FP64 path: the four products on the tensor cores
-        launch_fx_dst(c, (const double *)c.d_X, (double *)c.d_Y, c.d_h, g_begin, g_end, true);
     } else {
         // 1. DST along R
         stage_mark(c, 0);
@@ -1684,9 +1684,9 @@ void launch_hphi(Ctx &c, const double *psi, int g_begin, int g_end)
         // mixed path: j^2 + l^2 + Coriolis in one factorised tensor-core contraction
         launch_tc_ang(c, (const float *)c.d_X, c.d_h, g_begin, g_end, c.x_t);
         stage_mark(c, 4);
-    } else if (sizeof(T) == 8 && c.use_fx_ang) {
-        // FP64 path: the same contraction from exact digits; Y is free after the last transform
-        launch_fx_ang(c, (const double *)c.d_X, (double *)c.d_Y, c.d_h, g_begin, g_end);
+    } else if (c.use_fx_ang) {
+        // the same contraction from exact digits; Y is free after the last transform
+        launch_fx_ang<T>(c, (const T *)c.d_X, (T *)c.d_Y, c.d_h, g_begin, g_end);
         stage_mark(c, 4);
     } else if (c.na > 1) {
         dim3 gj(c.ncj, c.n1, ng);
@@ -2244,9 +2244,9 @@ static void noalloc_hphi(Ctx &c, const WaveTables &t, unsigned char *scratch, co
     dim3 gr((unsigned)((nrows + BM - 1) / BM), ((n2 + 1) / 2 + BN - 1) / BN);
     const bool rader = sizeof(T) == 8 && c.d_rd_tw;
     // the digit products, unless a folded length along r1 needs a second scratch rectangle
-    const bool fx = sizeof(T) == 8 && c.use_fx && !c.d_fxZ;
+    const bool fx = c.use_fx && !c.d_fxZ;
     if (fx) {
-        launch_fx_dst(c, (const double *)X, (double *)Y, H, g0, g1, false);
+        launch_fx_dst<T>(c, X, Y, H, g0, g1, false);
     } else {
         if (rader)
             k_dst_rows_rader<false><<<rd_grid(), 256, 0, c.stream>>>(d, (const double *)X, (double *)Y, nullptr,
@@ -2271,8 +2271,8 @@ static void noalloc_hphi(Ctx &c, const WaveTables &t, unsigned char *scratch, co
     LAUNCH_CHECK(c);
     if (sizeof(T) == 4 && c.use_tc_ang) {
         launch_tc_ang(c, (const float *)X, H, g0, g1, false);   // its own scratch, [r1][R]
-    } else if (sizeof(T) == 8 && c.use_fx_ang) {
-        launch_fx_ang(c, (const double *)X, (double *)Y, H, g0, g1);
+    } else if (c.use_fx_ang) {
+        launch_fx_ang<T>(c, X, Y, H, g0, g1);
     } else if (na > 1) {
         dim3 gj(c.ncj, n1, ng);
         k_ang_j<T><<<gj, 256, angj_smem(c, sizeof(T)), c.stream>>>(d, X, (const T *)c.d_xj2, H, c.d_tj_ptr, c.d_tj,

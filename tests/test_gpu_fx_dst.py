@@ -45,6 +45,43 @@ def test_hphi_against_the_oracle(shape_run, n1, n2, na, extra):
     p.close()
 
 
+# mixed shapes outside the fused chain (R or r1 too long) or its 64-angle kernel
+MIXED = [(24, 300, 4, {}), (140, 150, 3, {}), (33, 259, 70, {"Jtot": 2, "iommax": 2}), (256, 512, 3, {}),
+         (20, 300, 145, {"Jtot": 1, "iommax": 1, "iparity": -1}),
+         (40, 400, 20, {"nelecmax": 2, "lambdas": (0, 1), "Jtot": 2, "iommax": 2})]
+
+
+@pytest.mark.parametrize("n1,n2,na,extra", MIXED)
+def test_mixed_hphi_against_the_oracle(shape_run, n1, n2, na, extra):
+    run = shape_run(n1, n2, na, extra)
+    p, ref = Propagator(run, "mixed"), Oracle(run)
+    rng = np.random.default_rng([n1, n2])
+    for psi in (rng.uniform(-1, 1, run.ntot), run.psi0):
+        h, e = p.hphi(psi), ref.hphi(psi)
+        # FP32 vectors between exact products: the mixed path's bar
+        assert np.abs(h - e).max() <= 1e-6 * np.abs(e).max()
+    p.start()
+    ref.start(run.psi0)
+    p.run(40)
+    nrm = ref.run_iters(40)
+    assert np.abs(p.norms()[1:] - nrm).max() <= 1e-5 * np.abs(nrm).max()
+    p.close()
+
+
+@pytest.mark.parametrize("n1,n2,na,extra", [(48, 64, 66, {"nelecmax": 2}), (20, 34, 145, {"Jtot": 2, "iommax": 2})])
+@pytest.mark.parametrize("dst", [0, 3])
+def test_mixed_angular_form_beside_the_explicit_one(shape_run, n1, n2, na, extra, dst):
+    run = shape_run(n1, n2, na, extra)
+    want, err = Oracle(run).hphi(run.psi0), {}
+    for ang in (-1, 0):
+        p = Propagator(run, "mixed")
+        p.set_choices({"dst": dst, "angular": ang})
+        err[ang] = np.abs(p.hphi(run.psi0) - want).max() / np.abs(want).max()
+        p.close()
+    # no further off than the explicit FP32 sums, up to one rounding of the vectors kept in FP32
+    assert err[-1] <= err[0] + 2.0 ** -23
+
+
 def test_non_finite_input_stays_non_finite(shape_run):
     run = shape_run(24, 40, 4, {})
     p = Propagator(run, "fp64")
