@@ -835,13 +835,16 @@ int build_fx_ang_t(Ctx &c)
 
 }  // namespace
 
-// tables of the digit DSTs; leaves c.use_fx false where another path is asked for or faster
-// (mixed: the fused chain) or the shape is outside them
+// tables of the digit DSTs; leaves c.use_fx false where another path is asked for or the shape
+// is outside them.  Mixed: the fused chain is faster (one kernel, 2.6 against an estimated 4 ms
+// on the J = 0..40 sweep), and the three-kernel 3xTF32 form keeps its shapes (every r1 length up
+// to 128): results there would otherwise move by its own error, 2e-5 of psi after 32 iterations
+// at npun2 = 436; what is left ran on FP32 CUDA cores (512 x 256 x 120: 1.56 ms against 0.74)
 int build_fx(Ctx &c)
 {
     c.use_fx = false;
     c.d_fxZ = nullptr;
-    if (c.k_dst >= 0 || (!c.fp64 && c.use_tc_dst2d)) return MW3_OK;
+    if (c.k_dst >= 0 || (!c.fp64 && (c.use_tc_dst2d || tc_dst_supported(c)))) return MW3_OK;
     return c.fp64 ? build_fx_t<double>(c) : build_fx_t<float>(c);
 }
 

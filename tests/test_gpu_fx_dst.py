@@ -45,10 +45,10 @@ def test_hphi_against_the_oracle(shape_run, n1, n2, na, extra):
     p.close()
 
 
-# mixed shapes outside the fused chain (R or r1 too long) or its 64-angle kernel
-MIXED = [(24, 300, 4, {}), (140, 150, 3, {}), (33, 259, 70, {"Jtot": 2, "iommax": 2}), (256, 512, 3, {}),
-         (20, 300, 145, {"Jtot": 1, "iommax": 1, "iparity": -1}),
-         (40, 400, 20, {"nelecmax": 2, "lambdas": (0, 1), "Jtot": 2, "iommax": 2})]
+# mixed shapes whose r1 lengths pass one 128-row operand
+MIXED = [(150, 150, 3, {}), (256, 512, 2, {}), (145, 69, 70, {"Jtot": 2, "iommax": 2}),
+         (148, 50, 129, {"Jtot": 1, "iommax": 1, "iparity": -1}),
+         (160, 400, 6, {"nelecmax": 2, "lambdas": (0, 1), "Jtot": 2, "iommax": 2})]
 
 
 @pytest.mark.parametrize("n1,n2,na,extra", MIXED)
@@ -61,9 +61,10 @@ def test_mixed_hphi_against_the_oracle(shape_run, n1, n2, na, extra):
         # FP32 vectors between exact products: the mixed path's bar
         assert np.abs(h - e).max() <= 1e-6 * np.abs(e).max()
     p.start()
+    assert not p.path()["tc_dst"]
     ref.start(run.psi0)
-    p.run(40)
-    nrm = ref.run_iters(40)
+    p.run(20)
+    nrm = ref.run_iters(20)
     assert np.abs(p.norms()[1:] - nrm).max() <= 1e-5 * np.abs(nrm).max()
     p.close()
 
