@@ -73,6 +73,15 @@ void free_device(Ctx &c)
     c.built = false;
 }
 
+void drop_streams(Ctx &c)
+{
+    if (c.side) cudaStreamDestroy(c.side);
+    if (c.stream) cudaStreamDestroy(c.stream);
+    if (c.ev_upd) cudaEventDestroy(c.ev_upd);
+    for (cudaEvent_t e : c.ev_acc)
+        if (e) cudaEventDestroy(e);
+}
+
 #define TRY(x)                 \
     do {                       \
         int rc_ = (x);         \
@@ -536,7 +545,7 @@ int build_device(Ctx &c)
         c.n_upd_chunks = (int)ch.size();
         TRY(dupload(c, &c.d_upd_desc, ch));
     }
-    TRY(dalloc(c, &c.d_normpart, (size_t)c.nseg * c.nchunk));
+    TRY(dalloc(c, &c.d_normpart, (size_t)2 * c.nseg * c.nchunk));
     // ---- accumulators: context-wide arrays, each wave a slice ----
     {
         const WaveTables &t0 = c.waves[0];
@@ -968,6 +977,16 @@ int mw3_create(mw3_ctx **out, const mw3_grid *g, const int32_t *npunreal, const 
         if (e == cudaSuccess) *c.h_flag = 0;
         else cudaStreamDestroy(c.stream);
     }
+    if (e == cudaSuccess) {
+        // without them the iterations run in sequence on one stream
+        if (cudaEventCreateWithFlags(&c.ev_upd, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&c.ev_acc[0], cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&c.ev_acc[1], cudaEventDisableTiming) != cudaSuccess ||
+            cudaStreamCreateWithFlags(&c.side, cudaStreamNonBlocking) != cudaSuccess) {
+            cudaGetLastError();
+            c.side = nullptr;
+        }
+    }
     if (e != cudaSuccess) {
         delete h;
         return MW3_ERR_CUDA;
@@ -978,7 +997,7 @@ int mw3_create(mw3_ctx **out, const mw3_grid *g, const int32_t *npunreal, const 
         // the dynamic shared memory the kernels need must fit the device (the
         // explicit angular kernels narrow their column chunk for large angle counts)
         if (!mw3::fit_smem(c, prop.sharedMemPerBlockOptin)) {
-            cudaStreamDestroy(c.stream);
+            drop_streams(c);
             cudaFreeHost(c.h_flag);
             delete h;
             return MW3_ERR_UNSUPPORTED;
@@ -1122,19 +1141,47 @@ int mw3_upload_state(mw3_ctx *h, int32_t w, const double *psi_km1, const double 
 
 namespace {
 
-// one Chebyshev iteration of every wave, launched on the context's stream
+// the main stream waits for the accumulators of both parities
+void join_acc(Ctx &c)
+{
+    for (int p = 0; p < 2; p++) {
+        if (c.acc_open[p]) cudaStreamWaitEvent(c.stream, c.ev_acc[p], 0);
+        c.acc_open[p] = false;
+    }
+}
+
+// one Chebyshev iteration of every wave: H psi and the update on the context's stream, the
+// accumulators beside the next iteration's H psi (in sequence while stages are timed).  One
+// J = 0 wave leaves most SMs idle in both, and their launches add up: 78 us an iteration in
+// sequence, of which the accumulators 35
 void run_iteration(Ctx &c)
 {
     int64_t it = c.it + 1;
+    const int par = (int)(it & 1);
+    const bool beside = c.side && !c.prof;
     hphi_all(c, c.d_pk, 0, c.G);
     if (c.nofemax > 0) mw3::launch_fe_coef(c, it);
+    // psi_it overwrites psi_it-2 and its norm partials: its accumulators must be through
+    if (c.acc_open[par]) cudaStreamWaitEvent(c.stream, c.ev_acc[par], 0);
+    c.acc_open[par] = false;
+    c.norm_par = par;
     update(c, 0);
     std::swap(c.d_pk, c.d_pkm1);
     std::swap(c.d_pk32, c.d_pkm1_32);
+    if (beside) {
+        cudaEventRecord(c.ev_upd, c.stream);
+        cudaStreamWaitEvent(c.side, c.ev_upd, 0);
+        std::swap(c.stream, c.side);
+    }
     mw3::launch_accumulators(c, it);
     mw3::launch_norms(c, c.norm_slot);
     if (c.auto_nb > 0) mw3::launch_autocorr(c, c.norm_slot);
     mw3::launch_cvj_keep(c, it, c.norm_slot);
+    if (beside) {
+        cudaEventRecord(c.ev_acc[par], c.stream);
+        c.acc_open[par] = true;
+        std::swap(c.stream, c.side);
+    }
     if (c.hist_cap > 0) c.hist_n = std::min(c.hist_n + 1, c.hist_cap);
     if (c.prof && c.prof_n < c.prof_cap) {
         mw3::stage_mark(c, MW3_NSTAGES);
@@ -1180,6 +1227,7 @@ void capture_graph(Ctx &c, int par)
     c.cap_it0 = it0;
     c.cap_slot0 = slot0;
     for (int i = 0; i < mw3::kGraphIters; i++) run_iteration(c);
+    join_acc(c);
     c.capturing = false;
     cudaError_t e = cudaStreamEndCapture(c.stream, &g);
     const int64_t launches = c.launches - l0;
@@ -1227,6 +1275,7 @@ int mw3_run(mw3_ctx *h, int64_t n)
         if (graph_ready(c, n - s)) {
             // kGraphIters iterations as one graph replay
             const int par = c.d_pk == c.d_psiA ? 0 : 1;
+            join_acc(c);
             if (!c.graph_exec[par]) capture_graph(c, par);
             if (c.graph_exec[par]) {
                 mw3::launch_set_itbase(c);
@@ -1242,6 +1291,7 @@ int mw3_run(mw3_ctx *h, int64_t n)
         run_iteration(c);
         s++;
     }
+    join_acc(c);
     return check_launch(c, "mw3_run");
 }
 
@@ -1670,7 +1720,7 @@ int mw3_destroy(mw3_ctx *h)
     if (c.stream) cudaStreamSynchronize(c.stream);
     for (cudaEvent_t e : c.prof_ev) cudaEventDestroy(e);
     free_device(c);
-    if (c.stream) cudaStreamDestroy(c.stream);
+    drop_streams(c);
     if (c.h_flag) cudaFreeHost(c.h_flag);
     delete h;
     return MW3_OK;

@@ -136,6 +136,13 @@ struct Ctx {
     bool fp64;
     std::string err;
     cudaStream_t stream = nullptr;
+    // the accumulators, norms and records of an iteration run on a stream of their own beside the
+    // next iteration's H psi: they read psi_k, which the update after the next overwrites.  Every
+    // mw3_run (and every captured block) ends joined, so all other calls see one stream
+    cudaStream_t side = nullptr;
+    cudaEvent_t ev_upd = nullptr, ev_acc[2] = {nullptr, nullptr};
+    bool acc_open[2] = {false, false};   // accumulators of that parity not joined yet
+    int norm_par = 0;                // half of d_normpart the last update wrote
     int64_t launches = 0;
     bool started = false;
     int64_t it = 0;                  // Chebyshev index of psi_k (all waves advance together)
@@ -179,7 +186,7 @@ struct Ctx {
     double *d_psiA = nullptr, *d_psiB = nullptr;
     double *d_pk = nullptr, *d_pkm1 = nullptr;       // aliases, swapped every iteration
     double *d_h = nullptr;
-    double *d_normpart = nullptr;    // [G*na]
+    double *d_normpart = nullptr;    // [2][G*na][nchunk], by iteration parity
     // per-wave device tables
     int64_t *d_wflat0 = nullptr;     // [W+1]
     int *d_wseg0 = nullptr, *d_wseg1 = nullptr;      // segment range of each wave

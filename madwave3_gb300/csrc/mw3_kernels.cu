@@ -1728,7 +1728,7 @@ void launch_update(Ctx &c, int first)
     u.desc = c.d_upd_desc;
     u.nchunk = c.nchunk;
     u.first = first;
-    u.normpart = c.d_normpart;
+    u.normpart = c.d_normpart + (size_t)c.norm_par * c.nseg * c.nchunk;
     u.nofe = c.nofemax;
     u.zcke = c.d_zcke;
     u.zfe = c.d_zfe_ptrs;
@@ -2167,7 +2167,7 @@ void launch_set_itbase(Ctx &c)
 
 void launch_norms(Ctx &c, int64_t slot)
 {
-    k_norms<<<(int)c.waves.size(), 256, 0, c.stream>>>(c.d_normpart, c.d_wseg0, c.d_wseg1, c.nchunk,
+    k_norms<<<(int)c.waves.size(), 256, 0, c.stream>>>(c.d_normpart + (size_t)c.norm_par * c.nseg * c.nchunk, c.d_wseg0, c.d_wseg1, c.nchunk,
                                                        c.d_norm_ptrs, c.d_norm_cap,
                                                        c.capturing ? slot - c.cap_slot0 : slot,
                                                        c.capturing ? c.d_itbase : nullptr);
