@@ -26,10 +26,10 @@ struct alignas(16) Item {
     int seg;
     int v0;          // first vector: r1 row (transforms along R) or column (along r1)
     int mode;        // 0 whole, 1 even outputs (sums), 2 odd outputs (differences); bits 2..: 128-row block
-    int nn;          // the segment's r1 length
+    int nn;          // the segment's r1 length, or the r1 row of an angular tile
     int nks;         // K steps
-    int a[2];        // first K step of its matrix in the first and in the second transform
-    int nv;          // vectors
+    int a[2];        // its matrix in the first and in the second transform, in 256-byte units
+    int nv_m8;       // vectors | rows of its matrix planes (a multiple of 8) << 8
 };
 
 template <typename T>
@@ -41,8 +41,9 @@ struct Args {
     T *dst;
     const unsigned char *planes;
     int pass;                    // 0, 1: the first or the second transform along this axis
+    int nst;                     // stages of the ring of A
     int perm;                    // outputs stored even part first
-    const T *etab;               // along r1, first product: k-space factor [nn][n2], by etoff
+    const T *etab;               // along r1, first product: k-space factor [n2][nn], by etoff
     const int64_t *etoff;        // [W][na]
     int drop;                    // bits the first digit gives up (long sums along R)
     const int *blk_wave;
@@ -59,16 +60,16 @@ struct Args {
     int *err;
 };
 
-// eight consecutive numbers, zero from n on; vec: they start on 16 bytes
+// eight consecutive numbers, zero from n on; vec: they start on 32 bytes (one 256-bit load
+// takes a whole sector a lane: half the cache lines a load instruction touches)
 __device__ __forceinline__ void load8(const double *x, int n, bool vec, double (&v)[8])
 {
     if (vec && n >= 8) {
 #pragma unroll
-        for (int c = 0; c < 8; c += 2) {
-            const double2 d = *reinterpret_cast<const double2 *>(x + c);
-            v[c] = d.x;
-            v[c + 1] = d.y;
-        }
+        for (int c = 0; c < 8; c += 4)
+            asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
+                         : "=d"(v[c]), "=d"(v[c + 1]), "=d"(v[c + 2]), "=d"(v[c + 3])
+                         : "l"(x + c));
     } else {
 #pragma unroll
         for (int c = 0; c < 8; c++) v[c] = c < n ? x[c] : 0.0;
@@ -78,46 +79,41 @@ __device__ __forceinline__ void load8(const double *x, int n, bool vec, double (
 __device__ __forceinline__ void load8(const float *x, int n, bool vec, float (&v)[8])
 {
     if (vec && n >= 8) {
-#pragma unroll
-        for (int c = 0; c < 8; c += 4) {
-            const float4 d = *reinterpret_cast<const float4 *>(x + c);
-            v[c] = d.x;
-            v[c + 1] = d.y;
-            v[c + 2] = d.z;
-            v[c + 3] = d.w;
-        }
+        asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                     : "l"(x));
     } else {
 #pragma unroll
         for (int c = 0; c < 8; c++) v[c] = c < n ? x[c] : 0.f;
     }
 }
 
-__device__ __forceinline__ void store8(double *q, int n, bool vec, const double (&y)[8])
+__device__ __forceinline__ void store4(double *q, int n, bool vec, const double (&y)[4])
 {
-    if (vec && n >= 8) {
-#pragma unroll
-        for (int c = 0; c < 8; c += 2) *reinterpret_cast<double2 *>(q + c) = make_double2(y[c], y[c + 1]);
+    if (vec && n >= 4) {
+        asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};"
+                     :
+                     : "l"(q), "d"(y[0]), "d"(y[1]), "d"(y[2]), "d"(y[3])
+                     : "memory");
     } else {
 #pragma unroll
-        for (int c = 0; c < 8; c++)
+        for (int c = 0; c < 4; c++)
             if (c < n) q[c] = y[c];
     }
 }
 
-__device__ __forceinline__ void store8(float *q, int n, bool vec, const float (&y)[8])
+__device__ __forceinline__ void store4(float *q, int n, bool vec, const float (&y)[4])
 {
-    if (vec && n >= 8) {
-#pragma unroll
-        for (int c = 0; c < 8; c += 4)
-            *reinterpret_cast<float4 *>(q + c) = make_float4(y[c], y[c + 1], y[c + 2], y[c + 3]);
+    if (vec && n >= 4) {
+        *reinterpret_cast<float4 *>(q) = make_float4(y[0], y[1], y[2], y[3]);
     } else {
 #pragma unroll
-        for (int c = 0; c < 8; c++)
+        for (int c = 0; c < 4; c++)
             if (c < n) q[c] = y[c];
     }
 }
 
-// a barrier of the workers; true for all of them where any of them passes true
+// a barrier of the filling warps; true for all of them where any of them passes true
 __device__ __forceinline__ bool barrier_or(bool x)
 {
     uint32_t r;
@@ -127,7 +123,7 @@ __device__ __forceinline__ bool barrier_or(bool x)
         "barrier.cta.red.or.pred q, 1, %2, p;\n\t"
         "selp.u32 %0, 1, 0, q;\n\t}"
         : "=r"(r)
-        : "r"((uint32_t)x), "n"(WORKERS)
+        : "r"((uint32_t)x), "n"(FILL)
         : "memory");
     return r != 0;
 }
@@ -161,30 +157,48 @@ __device__ __forceinline__ void ang_values(const Args<T> &p, int g, int j, int r
     }
 }
 
-template <typename T, int EPI>
-__global__ void __launch_bounds__(WORKERS, 2) k_fx_dst(Args<T> p)
+// One persistent CTA per SM takes its tiles in turn, four roles at work on different tiles:
+// warps 0-7 load vectors, find each one's largest entry and write digits (two B blocks in
+// shared memory), warp 17 copies the matrix steps through a ring, warp 16 issues the MMAs (two
+// sets of accumulators in tensor memory), warps 8-15 put the sums together and store them.
+// With every warp of a CTA going through these phases in turn, two CTAs an SM, a tile of 32
+// FP64 vectors took 40 k cycles a CTA: 5 k for the loads, 7 k for the digits, 11 k for the
+// MMAs, 7-20 k for the way back.  The MMAs of a K step take 500 cycles; with the copies and
+// their waits on the issuing thread it was 1400.
+template <typename T, int EPI, bool FOLD>
+__global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
 {
     typedef typename Num<T>::Int Int;
     constexpr int ND = Num<T>::ND, NV = Num<T>::NV;
-    constexpr uint32_t ASTEP = Size<T>::ASTEP, BSTEP = Size<T>::BSTEP, BBYTES = Size<T>::BBYTES;
-    // eight vectors a warp; the WPG warps of a group of eight share its K
-    constexpr int NG = NV / 8, WPG = 8 / NG, KT = 32 * WPG, U = KB / KT;
+    constexpr uint32_t BSTEP = Size<T>::BSTEP, BBYTES = Size<T>::BBYTES, ABYTES = Size<T>::ABYTES;
+    // eight vectors a filling warp; the WPG warps of a group of eight share its K
+    constexpr int NG = NV / 8, WPG = FILL / 32 / NG, KT = 32 * WPG, U = KB / KT;
     constexpr bool ROWS = EPI == EPI_ROWS || EPI == EPI_GATHER, ANG = EPI == EPI_ANG_J || EPI == EPI_ANG_G;
+    static_assert(!ROWS || FOLD, "transforms along R are folded");
     extern __shared__ __align__(128) unsigned char sm[];
-    unsigned char *Bs = sm, *As = sm + BBYTES;
-    uint64_t *full = reinterpret_cast<uint64_t *>(sm + BBYTES + 2 * ASTEP);
-    uint64_t *empty = full + 2, *done = full + 4;
-    uint32_t *slot = reinterpret_cast<uint32_t *>(full + 5);
+    unsigned char *As = sm, *Bs = sm + ABYTES;
+    uint64_t *full = reinterpret_cast<uint64_t *>(sm + ABYTES + 2 * BBYTES);
+    uint64_t *empty = full + MAXST;           // the ring of A
+    uint64_t *bfull = empty + MAXST, *bempty = bfull + 2;      // the B blocks
+    uint64_t *tfull = bempty + 2, *tempty = tfull + 2;         // the accumulators
+    uint32_t *slot = reinterpret_cast<uint32_t *>(tempty + 2);
     volatile int *fail = reinterpret_cast<volatile int *>(slot + 1);
-    unsigned *s_max = reinterpret_cast<unsigned *>(slot + 2);      // [2 buffers][WPG][NV]
+    unsigned *s_max = reinterpret_cast<unsigned *>(slot + 2);      // [NEF][WPG][NV]: largest |x| of a tile's vectors
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (warp == 0) tc::tmem_alloc(slot, 256);
+    const int nst = p.nst;
+    const uint32_t astage = (ABYTES / nst) & ~127u;
+    if (warp == 0) tc::tmem_alloc(slot, 512);
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < nst; i++) {
             tc::mbar_init(&full[i], 1);
             tc::mbar_init(&empty[i], 1);
         }
-        tc::mbar_init(done, 1);
+        for (int i = 0; i < 2; i++) {
+            tc::mbar_init(&bfull[i], FILL / 32);
+            tc::mbar_init(&bempty[i], 1);
+            tc::mbar_init(&tfull[i], 1);
+            tc::mbar_init(&tempty[i], WAYBACK / 32);
+        }
         *fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -193,316 +207,401 @@ __global__ void __launch_bounds__(WORKERS, 2) k_fx_dst(Args<T> p)
     tc::fence_after_sync();
     const uint32_t tb = *slot;
     const int n2 = p.n2, n1 = p.n1;
-
-    // thread 0 also copies the matrix steps of every item in turn, two in flight, and issues their MMAs
-    int ci = blockIdx.x, cks = 0, cn = 0, ct = 0;      // the copies' item, step, steps of it, copies issued
-    int t = 0;                                         // steps issued
-    const unsigned char *ca = nullptr;
-    auto copy_next = [&]() {
-        if (ci >= p.nitems) return;
-        if (cks == 0) {
-            ca = p.planes + (int64_t)p.items[ci].a[p.pass] * ASTEP;
-            cn = p.items[ci].nks;
-        }
-        const int s = ct & 1;
-        tc::mbar_expect_tx(&full[s], ASTEP);
-        tc::bulk_g2s(As + s * ASTEP, ca + (int64_t)cks * ASTEP, ASTEP, &full[s]);
-        ct++;
-        if (++cks == cn) {
-            cks = 0;
-            ci += gridDim.x;
-        }
+    const bool vec = n2 % (32 / (int)sizeof(T)) == 0;     // rows start on 32 bytes
+    auto length = [&](const Item &it) { return ANG ? p.na : ROWS ? n2 : it.nn; };
+    // the largest entries' exponent field of vector n of the j-th tile
+    auto field = [&](int j, int n) {
+        const unsigned *sx = s_max + (j % NEF) * WPG * NV;
+        return (int)((WPG == 2 ? max(sx[n], sx[NV + n]) : sx[n]) >> Num<T>::EBITS);
     };
-    if (threadIdx.x == 0) {
-        copy_next();
-        copy_next();
-    }
-    const uint64_t a0 = tc::sdesc(tc::smem_u32(As), LBO, SBO), b0 = tc::sdesc(tc::smem_u32(Bs), LBO, SBO);
-    {
-        const int q4 = warp & 3;
-        const int m = q4 * 32 + lane;
-        const uint32_t trow = tb + ((uint32_t)(q4 * 32) << 16);
-        const int grp = warp % NG, hf = warp / NG;
-        const bool vec = n2 % (16 / (int)sizeof(T)) == 0;     // rows start on 16 bytes
-        int nd = 0, ni = 0;                       // B blocks written, items done
-        bool bad = false;
-        T kept[U][8];
-        // entry k of this thread's eight vectors
-        auto column = [&](const Item &it, int k, T (&v)[8]) {
-            if (EPI == EPI_ANG_G)
-                ang_values(p, it.seg, k, it.nn, it.v0 + 8 * grp, it.nv - 8 * grp, vec, v);
-            else if (EPI == EPI_ANG_J)
-                load8(p.src + (((size_t)it.seg * p.na + k) * n1 + it.nn) * n2 + it.v0 + 8 * grp, it.nv - 8 * grp, vec, v);
-            else
-                load8(p.src + ((size_t)it.seg * n1 + k) * n2 + it.v0 + 8 * grp, it.nv - 8 * grp, vec, v);
-        };
+
+    constexpr int MMA_WARP = (FILL + WAYBACK) / 32;
+    if (warp >= MMA_WARP) {
+        regs_down<REG_AUX>();
+        if (warp == MMA_WARP + 1 && lane == 0) {
+            // ---- the matrix steps of every tile in turn, nst in flight ----
+            int ct = 0, cs = 0, cph = 0;                   // copies issued; the next one's stage and phase
+            bool ok = true;
+            for (int i = blockIdx.x; i < p.nitems && ok; i += gridDim.x) {
+                const int n = p.items[i].nks;
+                const uint32_t cb = (uint32_t)(p.items[i].nv_m8 >> 8) * (ND * 32);
+                const unsigned char *ca = p.planes + (int64_t)p.items[i].a[p.pass] * 256;
+                for (int ks = 0; ks < n; ks++) {
+                    if (ct >= nst && !(ok = wait(&empty[cs], cph ^ 1, fail))) break;
+                    tc::mbar_expect_tx(&full[cs], cb);
+                    tc::bulk_g2s(As + cs * astage, ca + (int64_t)ks * cb, cb, &full[cs]);
+                    ct++;
+                    if (++cs == nst) {
+                        cs = 0;
+                        cph ^= 1;
+                    }
+                }
+            }
+            // no copy stays in flight
+            for (int c = max(0, ct - nst); c < ct; c++) tc::mbar_wait(&full[c % nst], (c / nst) & 1);
+        } else if (warp == MMA_WARP && lane == 0) {
+            // ---- the MMAs ----
+            const uint64_t a0 = tc::sdesc(tc::smem_u32(As), LBO, SBO), b0 = tc::sdesc(tc::smem_u32(Bs), LBO, SBO);
+            int t = 0, ts = 0, tph = 0;                    // steps issued; the next one's stage and phase
+            int nb = 0, ni = 0;
+            bool ok = (int)blockIdx.x < p.nitems && wait(&full[0], 0, fail);
+            int nks = ok ? p.items[blockIdx.x].nks : 0, m8 = ok ? p.items[blockIdx.x].nv_m8 >> 8 : 0;
+            for (int i = blockIdx.x; i < p.nitems && ok; i += gridDim.x, ni++) {
+                const int nx = i + (int)gridDim.x;
+                const bool more = nx < p.nitems;
+                const int nks2 = more ? p.items[nx].nks : 0, m82 = more ? p.items[nx].nv_m8 >> 8 : 0;
+                if (ni >= 2) ok = wait(&tempty[ni & 1], ((ni >> 1) - 1) & 1, fail);
+                const uint32_t d = tb + 256u * (ni & 1);
+                for (int ks = 0; ks < nks && ok; ks++) {
+                    if (ks % (KB / KS) == 0 && !(ok = wait(&bfull[nb & 1], (nb >> 1) & 1, fail))) break;
+                    const bool lastk = ks + 1 == nks;
+                    const int s = ts;
+                    t++;
+                    if (++ts == nst) {
+                        ts = 0;
+                        tph ^= 1;
+                    }
+                    tc::fence_after_sync();
+                    step<T>(d, a0 + (uint64_t)(s * (astage >> 4)), m8,
+                            b0 + (uint64_t)(((nb & 1) * BBYTES + (ks % (KB / KS)) * BSTEP) >> 4), ROWS ? 0 : 1, ks == 0,
+                            [&] {      // the next step's matrix
+                                if (!lastk || more) ok = wait(&full[ts], tph, fail);
+                            });
+                    tc::mma_commit(&empty[s]);
+                    if (lastk || (ks + 1) % (KB / KS) == 0) {
+                        tc::mma_commit(&bempty[nb & 1]);
+                        nb++;
+                    }
+                    if (lastk) tc::mma_commit(&tfull[ni & 1]);
+                }
+                nks = nks2;
+                m8 = m82;
+            }
+            // no MMA stays in flight
+            for (int c = max(0, t - nst); c < t; c++) tc::mbar_wait(&empty[c % nst], (c / nst) & 1);
+        }
+        __syncwarp();
+    } else if (warp >= FILL / 32) {
+        // ---- the way back: lane = output, half the tile's vectors a thread ----
+        regs_down<REG_WAY>();
+        const int q4 = warp & 3, half = (warp >> 2) & 1, m = q4 * 32 + lane;
+        const uint32_t lrow = tb + ((uint32_t)(q4 * 32) << 16);
+        int ni = 0;
+        Item nxt = {};
+        if ((int)blockIdx.x < p.nitems) nxt = p.items[blockIdx.x];
         for (int i = blockIdx.x; i < p.nitems; i += gridDim.x, ni++) {
-            const Item it = p.items[i];
+            const Item it = nxt;
+            if (i + (int)gridDim.x < p.nitems) nxt = p.items[i + gridDim.x];
             const int a = ANG ? 0 : it.seg % p.na;
             const int md = it.mode & 3, mt = it.mode >> 2;
-            const int L = ANG ? p.na : ROWS ? n2 : it.nn;
-            const int K = md ? (L + 1) >> 1 : L;
-            const int nv = it.nv;
-            const int sh = Num<T>::SH - (md ? 1 : 0) - p.drop;
-            // the exponent field of vector n's largest |x|
-            auto field = [&](const unsigned *sx, int n) {
-                return (int)((WPG == 2 ? max(sx[n], sx[NV + n]) : sx[n]) >> Num<T>::EBITS);
-            };
-            unsigned *sx = s_max + (ni & 1) * WPG * NV;
-            // ---- the largest |x| of each vector ----
-            if (ROWS) {
-                const int n = (lane & 7) + 8 * grp, part = (lane >> 3) + 4 * hf;
-                const T *x = p.src + ((size_t)it.seg * n1 + it.v0 + n) * n2;
-                unsigned mx = 0;
-                if (n < nv)
-                    for (int k = 8 * part; k < L; k += 8 * 4 * WPG) {
-                        T v[8];
-                        load8(x + k, L - k, vec, v);
+            const int L = length(it), nv = it.nv_m8 & 255;
+            const int sh = Num<T>::SH - (md ? 1 : 0) - p.drop + (ANG ? p.dexp : 0);
+            const int L2 = (L + 1) >> 1;                                // even outputs
+            const int out = 128 * mt + m;                               // index within its parity
+            const bool on = md == 0 ? out < L : out < (md == 1 ? L2 : L - L2);
+            const int k = md == 0 ? out : 2 * out + md - 1;             // the output itself
+            const int pos = md == 0 ? out : p.perm && !(L & 1) ? out + (md == 1 ? 0 : L2) : k;
+            const bool any = __any_sync(0xffffffffu, on);
+            const bool ok = wait(&tfull[ni & 1], (ni >> 1) & 1, fail);
+            if (!__all_sync(0xffffffffu, ok)) break;
+            tc::fence_after_sync();
+            const uint32_t trow = lrow + 256u * (ni & 1);
+            const int64_t fo = EPI == EPI_GATHER ? p.foff[it.seg]
+                               : EPI == EPI_ANG_G && on ? p.foff[(size_t)it.seg * p.na + out] : 0;
+            const T *et = EPI == EPI_COLS_E && on
+                              ? p.etab + p.etoff[p.blk_wave[it.seg / p.na] * p.na + a] + (size_t)it.v0 * it.nn + k : nullptr;
+            const int cend = min(nv, (half + 1) * (NV / 2));
+#pragma unroll 1
+            for (int c0 = half * (NV / 2); c0 < cend && any; c0 += 4) {
+                // what the stores need is on its way while the sums are put together
+                int idx[4];
+                T e[4];
+                if (EPI == EPI_GATHER || EPI == EPI_ANG_G) {
+                    const int *mp = EPI == EPI_GATHER ? p.mapT + ((size_t)a * n2 + k) * n1 + it.v0 + c0
+                                                      : p.map + ((size_t)out * n1 + it.nn) * n2 + it.v0 + c0;
 #pragma unroll
-                        for (int c = 0; c < 8; c++) mx = max(mx, mag(v[c]));
+                    for (int c = 0; c < 4; c++) idx[c] = on && c0 + c < nv ? mp[c] : -1;
+                }
+                if (EPI == EPI_COLS_E)
+#pragma unroll
+                    for (int c = 0; c < 4; c++) e[c] = on && c0 + c < nv ? et[(size_t)(c0 + c) * it.nn] : (T)0;
+                uint32_t v[ND][4];
+                load_groups(trow + c0, NV, v);
+                T y[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    uint32_t g[ND];
+#pragma unroll
+                    for (int q = 0; q < ND; q++) g[q] = v[q][c];
+                    y[c] = combine(g, field(ni, c0 + c), sh);
+                }
+                if (on) {
+                    if (EPI == EPI_ROWS) {
+                        T *q = p.dst + ((size_t)it.seg * n1 + it.v0 + c0) * n2 + pos;
+#pragma unroll
+                        for (int c = 0; c < 4; c++)
+                            if (c0 + c < nv) q[(size_t)c * n2] = y[c];
+                    } else if (EPI == EPI_GATHER) {
+                        double *h0 = p.H + fo;
+#pragma unroll
+                        for (int c = 0; c < 4; c++)
+                            if (idx[c] >= 0) h0[idx[c]] = (double)y[c];
+                    } else if (EPI == EPI_ANG_G) {
+                        // one writer per point: adds at L2, no load in the way
+                        double *h0 = p.H + fo;
+#pragma unroll
+                        for (int c = 0; c < 4; c++)
+                            if (idx[c] >= 0) atomicAdd(h0 + idx[c], (double)y[c]);
+                    } else {
+                        T *q = EPI == EPI_ANG_J
+                                   ? p.dst + (((size_t)it.seg * p.na + out) * n1 + it.nn) * n2 + it.v0 + c0
+                                   : p.dst + ((size_t)it.seg * n1 + pos) * n2 + it.v0 + c0;
+                        if (EPI == EPI_COLS_E)
+#pragma unroll
+                            for (int c = 0; c < 4; c++) y[c] *= e[c];
+                        store4(q, nv - c0, vec, y);
                     }
-                mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-                mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-                if (lane < 8) sx[hf * NV + n] = mx;
+                }
+                __syncwarp();
+            }
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) arrive(&tempty[ni & 1]);
+        }
+    } else {
+        // ---- vectors into digits ----
+        regs_up<REG_FILL>();
+        const int grp = warp % NG, hf = warp / NG;
+        const int rn = (lane & 7) + 8 * grp, rp = (lane >> 3) + 4 * hf;      // along R: this thread's row and k group
+        T kv[U][8], kw[FOLD ? U : 1][8];                      // entries of the first B block, and their mirrors
+        unsigned kmax[ROWS ? 1 : 8];                          // the largest |x| past the first block
+        // entry k of this thread's eight vectors (transforms along r1, angles)
+        auto column = [&](const Item &it, int k, T (&v)[8]) {
+            const int n = (it.nv_m8 & 255) - 8 * grp;
+            if (EPI == EPI_ANG_G)
+                ang_values(p, it.seg, k, it.nn, it.v0 + 8 * grp, n, vec, v);
+            else if (EPI == EPI_ANG_J)
+                load8(p.src + (((size_t)it.seg * p.na + k) * n1 + it.nn) * n2 + it.v0 + 8 * grp, n, vec, v);
+            else
+                load8(p.src + ((size_t)it.seg * n1 + k) * n2 + it.v0 + 8 * grp, n, vec, v);
+        };
+        // along R: entries k..k+7 of this thread's row, and their mirrors L-1-k downwards
+        auto row = [&](const Item &it, int L, int k, T (&v)[8], T (&w)[8]) {
+            const T *x = p.src + ((size_t)it.seg * n1 + it.v0 + rn) * n2;
+            load8(x + k, ((L + 1) >> 1) - k, vec, v);
+            const int e = L - 8 - k;
+            if (e >= 0) {
+                load8(x + e, 8, vec && e % (32 / (int)sizeof(T)) == 0, w);
             } else {
-                unsigned mx[8];
 #pragma unroll
-                for (int c = 0; c < 8; c++) mx[c] = 0;
-                // the first B block's entries stay in registers for their digits
+                for (int c = 0; c < 8; c++) w[c] = e + c >= 0 ? x[e + c] : (T)0;
+            }
+        };
+        // a tile's first B block into registers, and the largest entries past it
+        auto fetch = [&](const Item &it) {
+            const int L = length(it), md = it.mode & 3, K = md ? (L + 1) >> 1 : L;
+            if (ROWS) {
+                const bool on = rn < (it.nv_m8 & 255);
+                kmax[0] = 0;
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int k = 8 * (rp + 4 * WPG * u);
+#pragma unroll
+                    for (int c = 0; c < 8; c++) kv[u][c] = kw[FOLD ? u : 0][c] = (T)0;
+                    if (on && k < K) row(it, L, k, kv[u], kw[FOLD ? u : 0]);
+                }
+                if (on)
+#pragma unroll 1
+                    for (int k = KB + 8 * rp; k < K; k += 32 * WPG) {
+                        T v[8], w[8];
+                        row(it, L, k, v, w);
+#pragma unroll
+                        for (int c = 0; c < 8; c++) kmax[0] = max(kmax[0], max(mag(v[c]), mag(w[c])));
+                    }
+            } else {
+#pragma unroll
+                for (int c = 0; c < 8; c++) kmax[ROWS ? 0 : c] = 0;
 #pragma unroll
                 for (int u = 0; u < U; u++) {
                     const int k = lane + 32 * hf + KT * u;
-                    if (k < L) {
-                        column(it, k, kept[u]);
 #pragma unroll
-                        for (int c = 0; c < 8; c++) mx[c] = max(mx[c], mag(kept[u][c]));
+                    for (int c = 0; c < 8; c++) kv[u][c] = (T)0;
+                    if (k < K) column(it, k, kv[u]);
+                    if (FOLD) {
+#pragma unroll
+                        for (int c = 0; c < 8; c++) kw[u][c] = (T)0;
+                        if (md && k < K) column(it, L - 1 - k, kw[u]);
                     }
                 }
 #pragma unroll 1
-                for (int k = lane + 32 * hf + KB; k < L; k += KT) {
+                for (int k = lane + 32 * hf + KB; k < K; k += KT) {
                     T v[8];
                     column(it, k, v);
 #pragma unroll
-                    for (int c = 0; c < 8; c++) mx[c] = max(mx[c], mag(v[c]));
-                }
-                __syncwarp();
-#pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    const unsigned r = __reduce_max_sync(0xffffffffu, mx[c]);
-                    if (lane == c) sx[hf * NV + 8 * grp + c] = r;
+                    for (int c = 0; c < 8; c++) kmax[ROWS ? 0 : c] = max(kmax[ROWS ? 0 : c], mag(v[c]));
                 }
             }
-            tc::fence_before_sync();
-            if (barrier_or(bad)) break;           // every worker, or none
-            // ---- digits, one block of K at a time ----
-            for (int kb = 0; kb < K; kb += KB) {
-                const int kr = (min(K - kb, KB) + KS - 1) & ~(KS - 1);
-                if (ROWS) {
-                    const int n = (lane & 7) + 8 * grp;
-                    const int ef = field(sx, n);
-                    const T *x = p.src + ((size_t)it.seg * n1 + it.v0 + n) * n2;
-#pragma unroll 1
+        };
+        int nb = 0, ni = 0;                       // B blocks written, tiles done
+        bool bad = false;
+        Item nxt = {};
+        if ((int)blockIdx.x < p.nitems) {
+            nxt = p.items[blockIdx.x];
+            fetch(nxt);
+        }
+        for (int i = blockIdx.x; i < p.nitems; i += gridDim.x, ni++) {
+            const Item it = nxt;
+            const int md = it.mode & 3, L = length(it), K = md ? (L + 1) >> 1 : L;
+            const int nv = it.nv_m8 & 255;
+            const int sh = Num<T>::SH - (md ? 1 : 0) - p.drop;
+            // ---- the largest |x| of each vector ----
+            unsigned *sx = s_max + (ni % NEF) * WPG * NV;
+            if (ROWS) {
+                unsigned mx = kmax[0];
+#pragma unroll
+                for (int u = 0; u < U; u++)
+#pragma unroll
+                    for (int c = 0; c < 8; c++) mx = max(mx, max(mag(kv[u][c]), mag(kw[FOLD ? u : 0][c])));
+                mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+                mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+                if (lane < 8) sx[hf * NV + rn] = mx;
+            } else {
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    unsigned mx = kmax[ROWS ? 0 : c];
+#pragma unroll
                     for (int u = 0; u < U; u++) {
-                        const int kg = (lane >> 3) + 4 * hf + 4 * WPG * u, k = kb + 8 * kg;
+                        mx = max(mx, mag(kv[u][c]));
+                        if (FOLD) mx = max(mx, mag(kw[FOLD ? u : 0][c]));
+                    }
+                    mx = __reduce_max_sync(0xffffffffu, mx);
+                    if (lane == c) sx[hf * NV + 8 * grp + c] = mx;
+                }
+            }
+            if (barrier_or(bad)) break;           // every filling thread, or none
+            if (i + (int)gridDim.x < p.nitems) nxt = p.items[i + gridDim.x];
+            // ---- digits, one block of K at a time ----
+            for (int kb = 0; kb < K; kb += KB, nb++) {
+                const int kr = (min(K - kb, KB) + KS - 1) & ~(KS - 1);
+                unsigned char *Bb = Bs + (nb & 1) * BBYTES;
+                if (nb >= 2 && !bad) bad = !wait(&bempty[nb & 1], ((nb >> 1) - 1) & 1, fail);
+                tc::fence_after_sync();
+                if (kb > 0) {                     // a later block's entries, all on their way together
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const int k = ROWS ? kb + 8 * (rp + 4 * WPG * u) : kb + lane + 32 * hf + KT * u;
+                        if (k >= K) continue;
+                        if (!ROWS) column(it, k, kv[u]);
+                        else if (rn < nv) row(it, L, k, kv[u], kw[FOLD ? u : 0]);
+                    }
+                }
+                if (ROWS) {
+                    const int ef = field(ni, rn);
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const int kg = rp + 4 * WPG * u, k = kb + 8 * kg;
                         if (8 * kg >= kr) continue;
                         Int X[8];
 #pragma unroll
-                        for (int c = 0; c < 8; c++) X[c] = 0;
-                        if (n < nv && k < K) {
-                            T v[8], w[8];
-                            load8(x + k, K - k, vec, v);
-                            // x[L-1-k-c]: the eight entries that end at L - 1 - k, backwards
-                            const int e = L - 8 - k;
-                            if (e >= 0) load8(x + e, 8, vec && e % (16 / (int)sizeof(T)) == 0, w);
-                            else
-#pragma unroll
-                                for (int c = 0; c < 8; c++) w[c] = e + c >= 0 ? x[e + c] : (T)0;
-#pragma unroll
-                            for (int c = 0; c < 8; c++) {
-                                const int mr = L - 1 - (k + c);
-                                if (k + c >= K) continue;
-                                X[c] = to_fixed(v[c], ef, sh);
-                                const Int Y = mr != k + c ? to_fixed(w[7 - c], ef, sh) : md == 2 ? X[c] : 0;
+                        for (int c = 0; c < 8; c++) {
+                            X[c] = 0;
+                            if (rn < nv && k + c < K) {
+                                X[c] = to_fixed(kv[u][c], ef, sh);
+                                // the middle of an odd length pairs with itself
+                                const Int Y = L - 1 - (k + c) != k + c ? to_fixed(kw[FOLD ? u : 0][7 - c], ef, sh)
+                                                                       : md == 2 ? X[c] : 0;
                                 X[c] = md == 1 ? X[c] + Y : X[c] - Y;
                             }
                         }
-                        put_digits(X, Bs + (kg >> 1) * BSTEP + (n >> 3) * SBO + (kg & 1) * LBO + (n & 7) * 16,
+                        put_digits(X, Bb + (kg >> 1) * BSTEP + (rn >> 3) * SBO + (kg & 1) * LBO + (rn & 7) * 16,
                                    NV / 8 * SBO);
                     }
                 } else {
-                    int ef[8];
-#pragma unroll
-                    for (int c = 0; c < 8; c++)
-                        ef[c] = field(sx, 8 * grp + c);
 #pragma unroll
                     for (int u = 0; u < U; u++) {
                         const int kl = lane + 32 * hf + KT * u, k = kb + kl;
                         if (kl - lane >= kr) continue;
                         Int X[8];
 #pragma unroll
-                        for (int c = 0; c < 8; c++) X[c] = 0;
-                        if (k < K) {
-                            T v[8];
-                            if (kb == 0)
-#pragma unroll
-                                for (int c = 0; c < 8; c++) v[c] = kept[u][c];
-                            else
-                                column(it, k, v);
-#pragma unroll
-                            for (int c = 0; c < 8; c++) X[c] = to_fixed(v[c], ef[c], sh);
-                            if (md) {
-                                const int mr = L - 1 - k;
-                                if (mr != k) {
-                                    column(it, mr, v);
-#pragma unroll
-                                    for (int c = 0; c < 8; c++) {
-                                        const Int Y = to_fixed(v[c], ef[c], sh);
-                                        X[c] = md == 1 ? X[c] + Y : X[c] - Y;
-                                    }
-                                } else if (md == 2) {
-#pragma unroll
-                                    for (int c = 0; c < 8; c++) X[c] = 0;
+                        for (int c = 0; c < 8; c++) {
+                            const int ef = field(ni, 8 * grp + c);
+                            X[c] = 0;
+                            if (k < K) {
+                                X[c] = to_fixed(kv[u][c], ef, sh);
+                                if (FOLD && md) {
+                                    const Int Y =
+                                        L - 1 - k != k ? to_fixed(kw[FOLD ? u : 0][c], ef, sh) : md == 2 ? X[c] : 0;
+                                    X[c] = md == 1 ? X[c] + Y : X[c] - Y;
                                 }
                             }
                         }
-                        put_digits(X, Bs + (kl >> 4) * BSTEP + grp * SBO + ((kl >> 3) & 1) * LBO + (kl & 7) * 16,
+                        put_digits(X, Bb + (kl >> 4) * BSTEP + grp * SBO + ((kl >> 3) & 1) * LBO + (kl & 7) * 16,
                                    NV / 8 * SBO);
                     }
                 }
                 tc::fence_async_smem();
-                tc::fence_before_sync();
-                if (barrier_or(bad)) break;           // every worker, or none
-                if (threadIdx.x == 0) {
-                    tc::fence_after_sync();
-                    bool ok = true;
-                    for (int ks = 0; ks < kr / KS && ok; ks++) {
-                        const int s = t & 1;
-                        ok = wait(&full[s], (t >> 1) & 1, fail);
-                        if (!ok) break;
-                        step<T>(tb, a0 + (uint64_t)(s * (ASTEP >> 4)), b0 + (uint64_t)(ks * (BSTEP >> 4)), ROWS ? 0 : 1,
-                             kb + ks > 0);
-                        tc::mma_commit(&empty[s]);
-                        t++;
-                        // the next copy's stage was read two steps ago: wait for those MMAs, with
-                        // the step just issued running meanwhile
-                        if (ct <= t && ci < p.nitems && ks + 1 < kr / KS) {
-                            ok = wait(&empty[ct & 1], ((ct - 2) >> 1) & 1, fail);
-                            if (ok) copy_next();
-                        }
-                    }
-                    if (ok) tc::mma_commit(done);
-                }
                 __syncwarp();
-                bad = !wait(done, nd & 1, fail);
-                bad = __any_sync(0xffffffffu, bad);
-                tc::fence_after_sync();
-                nd++;
-                if (threadIdx.x == 0 && !bad)
-                    while (ct < t + 2 && ci < p.nitems) copy_next();
+                if (lane == 0 && !bad) arrive(&bfull[nb & 1]);
             }
-            bad = bad || *fail;
             bad = __any_sync(0xffffffffu, bad);
-            // ---- epilogue: lane = output, NV / 2 vectors a thread ----
-            const int L2 = (L + 1) >> 1;                                // even outputs
-            const int out = 128 * mt + m;                               // index within its parity
-            const bool on = !bad && (md == 0 ? out < L : out < (md == 1 ? L2 : L - L2));
-            const int k = md == 0 ? out : 2 * out + md - 1;             // the output itself
-            const int pos = md == 0 ? out : p.perm && !(L & 1) ? out + (md == 1 ? 0 : L2) : k;
-#pragma unroll 1
-            for (int h = 0; h < NV / 16; h++) {
-                const int c0 = (warp >> 2) * (NV / 2) + 8 * h;
-                uint32_t v[ND][8];
-                load_groups(trow + c0, NV, v);
-                if (on && c0 < nv) {
-                    T y[8];
-#pragma unroll
-                    for (int c = 0; c < 8; c++)
-                        y[c] = combine(v, c, field(sx, c0 + c), sh + (ANG ? p.dexp : 0));
-                    if (EPI == EPI_ROWS) {
-                        T *q = p.dst + ((size_t)it.seg * n1 + it.v0 + c0) * n2 + pos;
-#pragma unroll
-                        for (int c = 0; c < 8; c++)
-                            if (c0 + c < nv) q[(size_t)c * n2] = y[c];
-                    } else if (EPI == EPI_GATHER) {
-                        const int *mp = p.mapT + ((size_t)a * n2 + k) * n1 + it.v0 + c0;
-                        double *h0 = p.H + p.foff[it.seg];
-                        int idx[8];
-#pragma unroll
-                        for (int c = 0; c < 8; c++) idx[c] = c0 + c < nv ? mp[c] : -1;
-#pragma unroll
-                        for (int c = 0; c < 8; c++)
-                            if (idx[c] >= 0) h0[idx[c]] = (double)y[c];
-                    } else if (EPI == EPI_ANG_G) {
-                        // one writer per point: adds at L2, no load in the way
-                        const int *mp = p.map + ((size_t)out * n1 + it.nn) * n2 + it.v0 + c0;
-                        double *h0 = p.H + p.foff[(size_t)it.seg * p.na + out];
-                        int idx[8];
-#pragma unroll
-                        for (int c = 0; c < 8; c++) idx[c] = c0 + c < nv ? mp[c] : -1;
-#pragma unroll
-                        for (int c = 0; c < 8; c++)
-                            if (idx[c] >= 0) atomicAdd(h0 + idx[c], (double)y[c]);
-                    } else {
-                        T *q = EPI == EPI_ANG_J
-                                        ? p.dst + (((size_t)it.seg * p.na + out) * n1 + it.nn) * n2 + it.v0 + c0
-                                        : p.dst + ((size_t)it.seg * n1 + pos) * n2 + it.v0 + c0;
-                        if (EPI == EPI_COLS_E) {
-                            const int wa = p.blk_wave[it.seg / p.na] * p.na + a;
-                            T e[8];
-                            load8(p.etab + p.etoff[wa] + (size_t)k * n2 + it.v0 + c0, nv - c0, vec, e);
-#pragma unroll
-                            for (int c = 0; c < 8; c++) y[c] *= e[c];
-                        }
-                        store8(q, nv - c0, vec, y);
-                    }
-                }
-                __syncwarp();
-            }
+            if (i + (int)gridDim.x < p.nitems) fetch(nxt);
         }
-    }
-    if (threadIdx.x == 0) {                       // nothing of this thread's stays in flight
-        for (int c = max(0, ct - 2); c < ct; c++) tc::mbar_wait(&full[c & 1], (c >> 1) & 1);
-        for (int c = max(0, t - 2); c < t; c++) tc::mbar_wait(&empty[c & 1], (c >> 1) & 1);
     }
     tc::fence_before_sync();
     __syncthreads();
     if (threadIdx.x == 0 && *fail) atomicExch(p.err, 1);
-    if (warp == 0) tc::tmem_dealloc(tb, 256);
+    if (warp == 0) tc::tmem_dealloc(tb, 512);
 }
 
 }  // namespace fx
 
 namespace {
 
-// digits of the rows of one constant matrix, columns col(q), as K steps of 128-row planes
-// (canonical K-major), appended to `out`.  Returns the bits a vector's first digit (up to
+// rows of the planes of a matrix of M rows (of each of its 128-row blocks)
+inline int plane_rows(int M) { return std::min(128, (M + 7) & ~7); }
+
+// bytes of one K step of them, in the 256-byte units of a tile's matrix index
+template <typename T>
+int step_units(int m8) { return fx::Num<T>::ND * m8 / 8; }
+
+// stages of the ring of A for planes of up to m8 rows
+template <typename T>
+int ring_stages(int m8)
+{
+    int n = fx::MAXST;
+    while (((fx::Size<T>::ABYTES / n) & ~127u) < (uint32_t)step_units<T>(m8) * 256) n--;
+    return n;
+}
+
+// digits of the rows of one constant matrix as K steps of planes of m8 rows (canonical
+// K-major), one 128-row block after the other, appended to `out`.  Returns the bits a vector's first digit (up to
 // 512, or 64 of FP32) has to give up so that no group g <= 4 of a row can sum past 2^24.
 // value(m, k): the entry x 2^SBITS, an integer of at most 2^(SBITS+1)
 template <typename T, typename F>
-int append_planes(std::vector<__half> &out, int M, int K, F &&value)
+int append_planes(std::vector<__half> &out, int M, int m8, int K, F &&value)
 {
     constexpr int ND = fx::Num<T>::ND;
-    constexpr uint32_t ASTEP = fx::Size<T>::ASTEP;
     static const std::vector<__half> half_of = [] {
         std::vector<__half> h(513);
         for (int d = 0; d <= 512; d++) h[d] = __float2half((float)(d - 256));
         return h;
     }();
     const double first = sizeof(T) == 8 ? 512.0 : 64.0;       // a vector's first digit
-    const int nks = (K + fx::KS - 1) / fx::KS, nmt = (M + 127) / 128;
-    const size_t base = out.size();
-    out.resize(base + (size_t)nmt * nks * ASTEP / 2, half_of[256]);
+    const int nks = (K + fx::KS - 1) / fx::KS;
+    const int nmt = (M + 127) / 128;
+    const size_t base = out.size(), plane = (size_t)m8 * fx::KS, ast = ND * plane;
+    out.resize(base + (size_t)nmt * nks * ast, half_of[256]);
     int drop = 0;
     for (int m = 0; m < M; m++) {
         long long sum[ND] = {};                 // of |digit| over k
         for (int k = 0; k < K; k++) {
             long long v = value(m, k);
-            __half *st = out.data() + base +
-                         (((size_t)(m / 128) * nks + k / fx::KS) * ASTEP + fx::a_off(m % 128, k % fx::KS)) / 2;
+            __half *st = out.data() + base + ((size_t)(m / 128) * nks + k / fx::KS) * ast +
+                         fx::a_off(m % 128, k % fx::KS) / 2;
             for (int d = ND - 1; d >= 0; d--) {
                 const int g = d > 0 ? (int)((v + 128) & 255) - 128 : (int)v;
                 v = (v - g) >> 8;
-                st[(size_t)d * (fx::APL / 2)] = half_of[g + 256];
+                st[d * plane] = half_of[g + 256];
                 sum[d] += g < 0 ? -g : g;
             }
         }
@@ -532,13 +631,13 @@ struct Sine {
     long long operator()(int i, int k) const { return s[(long long)(i + 1) * (k + 1) % (2 * (n + 1))]; }
 };
 
-// resident CTAs of the persistent kernel: two per SM
+// resident CTAs of the persistent kernel: one per SM
 int fx_ctas()
 {
     int dev = 0, nsm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    return 2 * nsm;
+    return nsm;
 }
 
 template <typename V>
@@ -557,16 +656,16 @@ int fx_upload(Ctx &c, V **dst, const std::vector<V> &v)
     return MW3_OK;
 }
 
-template <typename T, int EPI>
+template <typename T, int EPI, bool FOLD>
 void set_smem()
 {
-    cudaFuncSetAttribute(fx::k_fx_dst<T, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fx::Size<T>::SMEM);
+    cudaFuncSetAttribute(fx::k_fx_dst<T, EPI, FOLD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fx::Size<T>::SMEM);
 }
 
-template <typename T, int EPI>
+template <typename T, int EPI, bool FOLD>
 void launch(Ctx &c, const fx::Args<T> &p)
 {
-    fx::k_fx_dst<T, EPI><<<std::min(p.nitems, c.fx_grid), fx::WORKERS, fx::Size<T>::SMEM, c.stream>>>(p);
+    fx::k_fx_dst<T, EPI, FOLD><<<std::min(p.nitems, c.fx_grid), fx::THREADS, fx::Size<T>::SMEM, c.stream>>>(p);
     c.launches++;
 }
 
@@ -574,7 +673,6 @@ template <typename T>
 int build_fx_t(Ctx &c)
 {
     constexpr int NV = fx::Num<T>::NV;
-    constexpr uint32_t ASTEP = fx::Size<T>::ASTEP;
     c.use_fx = false;
     c.d_fxZ = nullptr;
     // K of one product is at most 256: npun2 <= 512 folded, npun1 <= 256 (which mw3_create asks for)
@@ -584,17 +682,17 @@ int build_fx_t(Ctx &c)
     // along R: [pass][parity][128-row block][K step]
     {
         const Sine<T> S(n2);
-        const int he = (n2 + 1) / 2, ho = n2 / 2, K = he;
+        const int he = (n2 + 1) / 2, ho = n2 / 2, K = he, m8 = plane_rows(he);
         const bool perm = n2 % 2 == 0;
         for (int pass = 0; pass < 2; pass++) {
             std::vector<__half> pl;
             auto col = [&](int q) { return pass && perm ? 2 * q : q; };
             for (int par = 0; par < 2; par++) {
                 const size_t b = pl.size();
-                dropR = std::max(dropR, append_planes<T>(pl, par ? ho : he, K,
+                dropR = std::max(dropR, append_planes<T>(pl, par ? ho : he, m8, K,
                                                       [&](int m, int k) { return S(2 * m + par, col(k)); }));
                 // both parities take the even one's block count
-                const size_t want = (size_t)((he + 127) / 128) * ((K + fx::KS - 1) / fx::KS) * ASTEP / 2;
+                const size_t want = (size_t)((he + 127) / 128) * ((K + fx::KS - 1) / fx::KS) * step_units<T>(m8) * 128;
                 pl.resize(b + want, __float2half(0.f));
             }
             __half *d = nullptr;
@@ -623,14 +721,14 @@ int build_fx_t(Ctx &c)
                     std::pair<int64_t, int64_t> o;
                     o.first = o.second = (int64_t)pl.size() * 2;
                     if (nn <= 128) {
-                        drop1 = std::max(drop1, append_planes<T>(pl, nn, nn, [&](int m, int k) { return S(m, k); }));
+                        drop1 = std::max(drop1, append_planes<T>(pl, nn, plane_rows(nn), nn, [&](int m, int k) { return S(m, k); }));
                     } else {
                         fold = true;
                         const int K = (nn + 1) / 2;
                         for (int pass = 0; pass < (nn % 2 ? 1 : 2); pass++) {
                             if (pass) o.second = (int64_t)pl.size() * 2;
                             for (int par = 0; par < 2; par++)
-                                drop1 = std::max(drop1, append_planes<T>(pl, par ? nn / 2 : K, K, [&](int m, int k) {
+                                drop1 = std::max(drop1, append_planes<T>(pl, par ? nn / 2 : K, plane_rows(K), K, [&](int m, int k) {
                                                      return S(2 * m + par, pass ? 2 * k : k);
                                                  }));
                         }
@@ -638,17 +736,18 @@ int build_fx_t(Ctx &c)
                     // min(p1 + p2, radcut) / (4 (nn+1) (n2+1)) by stored column; the momenta depend on the length only
                     const int64_t eo = (int64_t)et.size();
                     const double divi = 1.0 / (4.0 * (double)(nn + 1) * (double)(n2 + 1));
-                    for (int m = 0; m < nn; m++)
-                        for (int q = 0; q < n2; q++) {
-                            const int R = n2 % 2 ? q : (q < he ? 2 * q : 2 * (q - he) + 1);
+                    for (int q = 0; q < n2; q++) {
+                        const int R = n2 % 2 ? q : (q < he ? 2 * q : 2 * (q - he) + 1);
+                        for (int m = 0; m < nn; m++) {
                             double ek = t.p2r1[(size_t)a * n1 + m] + t.p2r2[(size_t)a * n2 + R];
                             if (ek > c.grid.radcutmax) ek = c.grid.radcutmax;
                             et.push_back((T)(ek * divi));
                         }
+                    }
                     f = at.emplace(nn, std::make_pair(o, eo)).first;
                 }
-                off1[(size_t)w * na + a] = (int)(f->second.first.first / ASTEP);
-                off2[(size_t)w * na + a] = (int)(f->second.first.second / ASTEP);
+                off1[(size_t)w * na + a] = (int)(f->second.first.first / 256);
+                off2[(size_t)w * na + a] = (int)(f->second.first.second / 256);
                 eoff[(size_t)w * na + a] = f->second.second;
             }
         if (dropR > 1 || drop1 > 0) return MW3_OK;
@@ -679,6 +778,8 @@ int build_fx_t(Ctx &c)
     c.h_fx_row0.assign(1, 0);
     c.h_fx_col0.assign(1, 0);
     const int he = (n2 + 1) / 2, nmt = (he + 127) / 128, nmto = (n2 / 2 + 127) / 128, ksR = (he + fx::KS - 1) / fx::KS;
+    const int mR = plane_rows(he), uR = ksR * step_units<T>(mR);
+    int m1max = 8;
     for (int w = 0; w < W; w++)
         for (int b = 0; b < c.waves[w].ncan; b++)
             for (int a = 0; a < na; a++) {
@@ -687,28 +788,34 @@ int build_fx_t(Ctx &c)
                 for (int v = 0; v < nn; v += NV)
                     for (int par = 0; par < 2; par++)
                         for (int mt = 0; mt < (par ? nmto : nmt); mt++) {
-                            const int at = (par * nmt + mt) * ksR;
+                            const int at = (par * nmt + mt) * uR;
                             rows.push_back(fx::Item{seg, v, (par + 1) | (mt << 2), nn, ksR, {at, at},
-                                                    std::min((int)NV, nn - v)});
+                                                    std::min(NV, nn - v) | (mR << 8)});
                         }
-                const int K1 = nn <= 128 ? nn : (nn + 1) / 2, ks1 = (K1 + fx::KS - 1) / fx::KS;
+                const int K1 = nn <= 128 ? nn : (nn + 1) / 2, ks1 = (K1 + fx::KS - 1) / fx::KS, m1 = plane_rows(K1);
+                const int u1 = ks1 * step_units<T>(m1);
+                m1max = std::max(m1max, m1);
                 for (int v = 0; v < n2; v += NV)
                     for (int par = 0; par < (nn <= 128 ? 1 : 2); par++)
-                        cols.push_back(fx::Item{seg, v, nn <= 128 ? 0 : par + 1, nn, ks1,
-                                                {o1 + par * ks1, o2 + par * ks1}, std::min((int)NV, n2 - v)});
+                        cols.push_back(fx::Item{seg, v, nn <= 128 ? 0 : par + 1, nn, ks1, {o1 + par * u1, o2 + par * u1},
+                                                std::min(NV, n2 - v) | (m1 << 8)});
                 c.h_fx_row0.push_back((int)rows.size());
                 c.h_fx_col0.push_back((int)cols.size());
             }
+    c.fx_nst[0] = ring_stages<T>(mR);
+    c.fx_nst[1] = ring_stages<T>(m1max);
     fx::Item *d;
     int rc;
     if ((rc = fx_upload(c, &d, rows))) return rc;
     c.d_fx_rows = d;
     if ((rc = fx_upload(c, &d, cols))) return rc;
     c.d_fx_cols = d;
-    set_smem<T, fx::EPI_ROWS>();
-    set_smem<T, fx::EPI_GATHER>();
-    set_smem<T, fx::EPI_COLS_E>();
-    set_smem<T, fx::EPI_COLS>();
+    set_smem<T, fx::EPI_ROWS, true>();
+    set_smem<T, fx::EPI_GATHER, true>();
+    set_smem<T, fx::EPI_COLS_E, false>();
+    set_smem<T, fx::EPI_COLS, false>();
+    set_smem<T, fx::EPI_COLS_E, true>();
+    set_smem<T, fx::EPI_COLS, true>();
     c.fx_grid = fx_ctas();
     c.use_fx = true;
     return MW3_OK;
@@ -722,9 +829,9 @@ template <typename T>
 int build_fx_ang_t(Ctx &c)
 {
     constexpr int NV = fx::Num<T>::NV;
-    constexpr uint32_t ASTEP = fx::Size<T>::ASTEP;
     const int na = c.na, n1 = c.n1, n2 = c.n2, G = c.G, ne = c.ne;
-    const int nks = (na + fx::KS - 1) / fx::KS, nmt = (na + 127) / 128;
+    const int nks = (na + fx::KS - 1) / fx::KS, nmt = (na + 127) / 128, m8 = plane_rows(na);
+    const int units = nks * step_units<T>(m8);
     double dmax = 0.0;
     for (auto &t : c.waves)
         for (double d : t.djmmp) {
@@ -758,16 +865,16 @@ int build_fx_ang_t(Ctx &c)
                 f = (int)seen.size();
                 seen.push_back(D);
                 seen_lad.push_back(lad);
-                seen_at.push_back((int)(pl.size() * 2 / ASTEP));
+                seen_at.push_back((int)(pl.size() / 128));
                 auto d = [&](int js, int a) {
                     return js < njl ? llrint(ldexp(D[(size_t)(t.j0 + js * t.inc) * na + a], dexp + fx::Num<T>::SBITS))
                                     : 0LL;
                 };
-                drop = std::max(drop, append_planes<T>(pl, na, na, [&](int m, int k) { return d(m, k); }));
-                drop = std::max(drop, append_planes<T>(pl, na, na, [&](int m, int k) { return d(k, m); }));
+                drop = std::max(drop, append_planes<T>(pl, na, m8, na, [&](int m, int k) { return d(m, k); }));
+                drop = std::max(drop, append_planes<T>(pl, na, m8, na, [&](int m, int k) { return d(k, m); }));
             }
             at[2 * g] = seen_at[f];
-            at[2 * g + 1] = seen_at[f] + nmt * nks;
+            at[2 * g + 1] = seen_at[f] + nmt * units;
             // yyy of the block's own j list, by ladder slot
             for (int k = 0; k < t.nojbas[b]; k++) {
                 const int jb = t.jbas[(size_t)b * na + k];
@@ -808,8 +915,8 @@ int build_fx_ang_t(Ctx &c)
             for (int j = 0; j < t2n; j++)
                 if (on[(size_t)i * t2n + j])
                     for (int mt = 0; mt < nmt; mt++)
-                        items.push_back(fx::Item{g, j * NV, mt << 2, i, nks, {at[2 * g] + mt * nks, at[2 * g + 1] + mt * nks},
-                                                 std::min((int)NV, n2 - j * NV)});
+                        items.push_back(fx::Item{g, j * NV, mt << 2, i, nks, {at[2 * g] + mt * units, at[2 * g + 1] + mt * units},
+                                                 std::min(NV, n2 - j * NV) | (m8 << 8)});
         c.h_fx_ang0.push_back((int)items.size());
     }
     int rc;
@@ -824,10 +931,11 @@ int build_fx_ang_t(Ctx &c)
     c.d_fx_l2 = dl;
     c.d_fx_ang = di;
     c.d_fxD = d;
+    c.fx_nst[2] = ring_stages<T>(m8);
     c.fx_drop_ang = drop;
     c.fx_dexp = dexp;
-    set_smem<T, fx::EPI_ANG_J>();
-    set_smem<T, fx::EPI_ANG_G>();
+    set_smem<T, fx::EPI_ANG_J, false>();
+    set_smem<T, fx::EPI_ANG_G, false>();
     c.fx_grid = fx_ctas();
     c.use_fx_ang = true;
     return MW3_OK;
@@ -866,13 +974,13 @@ void launch_fx_ang(Ctx &c, const T *X, T *Y, double *H, int g_begin, int g_end)
     p.err = c.d_tc_err;
     p.planes = (const unsigned char *)c.d_fxD;
     p.yj = (const T *)c.d_fx_yj; p.l2 = (const T *)c.d_fx_l2; p.cpl = c.d_cpl;
-    p.drop = c.fx_drop_ang; p.dexp = c.fx_dexp;
+    p.drop = c.fx_drop_ang; p.dexp = c.fx_dexp; p.nst = c.fx_nst[2];
     p.items = (const fx::Item *)c.d_fx_ang + c.h_fx_ang0[g_begin];
     p.nitems = c.h_fx_ang0[g_end] - c.h_fx_ang0[g_begin];
     p.src = X; p.dst = Y; p.pass = 0;
-    launch<T, fx::EPI_ANG_J>(c, p);
+    launch<T, fx::EPI_ANG_J, false>(c, p);
     p.src = Y; p.dst = nullptr; p.pass = 1;
-    launch<T, fx::EPI_ANG_G>(c, p);
+    launch<T, fx::EPI_ANG_G, false>(c, p);
 }
 
 // the four products of the radial kinetic term of blocks [g_begin, g_end): X -> Y, Y in place
@@ -893,18 +1001,23 @@ void launch_fx_dst(Ctx &c, const T *X, T *Y, double *H, int g_begin, int g_end, 
     if (mark) stage_mark(c, 0);
     p.items = rows; p.nitems = nr;
     p.src = X; p.dst = Y; p.planes = (const unsigned char *)c.d_fxR[0]; p.perm = 1; p.pass = 0; p.drop = c.fx_drop;
-    launch<T, fx::EPI_ROWS>(c, p);
+    p.nst = c.fx_nst[0];
+    launch<T, fx::EPI_ROWS, true>(c, p);
     if (mark) stage_mark(c, 1);
     T *Z = c.d_fxZ ? (T *)c.d_fxZ : Y;
     p.items = cols; p.nitems = nc;
     p.src = Y; p.dst = Z; p.planes = (const unsigned char *)c.d_fxr; p.drop = 0;
-    launch<T, fx::EPI_COLS_E>(c, p);
+    p.nst = c.fx_nst[1];
+    if (c.d_fxZ) launch<T, fx::EPI_COLS_E, true>(c, p);
+    else launch<T, fx::EPI_COLS_E, false>(c, p);
     p.src = Z; p.dst = Y; p.perm = 0; p.pass = 1;
-    launch<T, fx::EPI_COLS>(c, p);
+    if (c.d_fxZ) launch<T, fx::EPI_COLS, true>(c, p);
+    else launch<T, fx::EPI_COLS, false>(c, p);
     if (mark) stage_mark(c, 2);
     p.items = rows; p.nitems = nr;
     p.src = Y; p.dst = nullptr; p.planes = (const unsigned char *)c.d_fxR[1]; p.drop = c.fx_drop;
-    launch<T, fx::EPI_GATHER>(c, p);
+    p.nst = c.fx_nst[0];
+    launch<T, fx::EPI_GATHER, true>(c, p);
 }
 
 template void launch_fx_dst<double>(Ctx &, const double *, double *, double *, int, int, bool);

@@ -22,11 +22,18 @@ constexpr int KS = 16;                             // K of one MMA
 constexpr int KB = 128;                            // K of one B block in shared memory
 constexpr uint32_t APL = 128 * KS * 2;             // one digit of one K step of A: 4 KB
 constexpr uint32_t SBO = 256, LBO = 128;
-constexpr int WORKERS = 256;
+constexpr int FILL = 256;                          // threads that cut vectors into digits: warps 0-7
+constexpr int WAYBACK = 256;                       // and that put the sums together: warps 8-15
+constexpr int THREADS = FILL + WAYBACK + 128;      // and one warp for the MMAs, one for the copies
+// registers a thread: 96 at launch (640 threads), then shared out by warpgroup: 256 x 128 +
+// 256 x 80 + 128 x 64 = 61440, all that the CTA was launched with
+constexpr int REG_FILL = 128, REG_WAY = 80, REG_AUX = 64;
+static_assert(FILL * REG_FILL + WAYBACK * REG_WAY + 128 * REG_AUX <= THREADS * 96, "more registers than at launch");
+constexpr int NEF = 8;                             // tiles whose exponents are kept (up to five are under way)
 
 // What depends on the type of the vectors.  FP32 vectors take four digits of 30 bits
 // (|X| <= 2^30, the constant matrix x 2^29), FP64 vectors seven; the accumulators of all
-// groups of one tile fill up to 256 tensor-memory columns, so two CTAs share an SM.
+// groups of one tile take up to 256 tensor-memory columns, half of them.
 template <typename T> struct Num;
 template <> struct Num<double> {
     enum { ND = 7, NV = 32, SH = 4, EBITS = 20, EMAX = 0x7FF, SBITS = 54 };
@@ -37,11 +44,12 @@ template <> struct Num<float> {
     typedef int Int;
 };
 template <typename T> struct Size {
-    static constexpr uint32_t ASTEP = Num<T>::ND * APL;                            // 28 or 16 KB
+    static constexpr uint32_t ABYTES = sizeof(T) == 8 ? 114688 : 98304;            // the ring of K steps of A
     static constexpr uint32_t BSTEP = Num<T>::ND * Num<T>::NV * KS * 2;            // 7 or 8 KB
-    static constexpr uint32_t BBYTES = (KB / KS) * BSTEP;                          // 56 or 64 KB
-    static constexpr uint32_t SMEM = BBYTES + 2 * ASTEP + 1024;                    // 113 or 97 KB
+    static constexpr uint32_t BBYTES = (KB / KS) * BSTEP;                          // 56 or 64 KB, twice
+    static constexpr uint32_t SMEM = ABYTES + 2 * BBYTES + 3072;                   // 227 KB: one CTA an SM
 };
+constexpr int MAXST = 8;                           // stages of the ring
 
 // element (row, k) of one digit of a K step of A
 __host__ __device__ constexpr uint32_t a_off(int r, int k)
@@ -137,13 +145,14 @@ __device__ __forceinline__ void put_digits(const int *X, unsigned char *dst, uin
     }
 }
 
-// one accumulator row of eight vectors: v[g][c], g the group; the sum over k of S x.
-// ef: exponent field of the vector's largest |x|, sh as in to_fixed
-__device__ __forceinline__ double combine(const uint32_t (&v)[7][8], int c, int ef, int sh)
+// one output: its seven groups -> the sum over k of S x.  ef: exponent field of the vector's
+// largest |x|, sh as in to_fixed.  (Conversions by FP32 additions and integer instructions
+// instead of the quarter-rate and FP64 units were no faster.)
+__device__ __forceinline__ double combine(const uint32_t (&v)[7], int ef, int sh)
 {
     int a[7];
 #pragma unroll
-    for (int g = 0; g < 7; g++) a[g] = __float2int_rn(__uint_as_float(v[g][c]));
+    for (int g = 0; g < 7; g++) a[g] = __float2int_rn(__uint_as_float(v[g]));
     const long long H = ((long long)a[0] << 24) + ((long long)a[1] << 16) + ((long long)a[2] << 8) + a[3];
     const long long L = ((long long)a[4] << 16) + ((long long)a[5] << 8) + a[6];
     // the leading 62 bits of H 2^24 + L, in units 2^(72-z) of 2^54 2^(57-E)
@@ -160,11 +169,11 @@ __device__ __forceinline__ double combine(const uint32_t (&v)[7][8], int c, int 
 }
 
 // the groups are exact; their FP32 sum rounds once at the size of the first
-__device__ __forceinline__ float combine(const uint32_t (&v)[4][8], int c, int ef, int sh)
+__device__ __forceinline__ float combine(const uint32_t (&v)[4], int ef, int sh)
 {
     const float r = 1.f / 256.f;
-    const float f = fmaf(fmaf(fmaf(__uint_as_float(v[3][c]), r, __uint_as_float(v[2][c])), r, __uint_as_float(v[1][c])),
-                         r, __uint_as_float(v[0][c]));
+    const float f = fmaf(fmaf(fmaf(__uint_as_float(v[3]), r, __uint_as_float(v[2])), r, __uint_as_float(v[1])), r,
+                         __uint_as_float(v[0]));
     if (ef >= 0xFF) return __uint_as_float(0x7FC00000u);
     const int sc = ef - 137 + (6 - sh);              // E - 11 (48 - 29 - 30), one more for a folded vector
     const int s0 = max(sc, -100);
@@ -199,6 +208,11 @@ __device__ __forceinline__ bool wait(uint64_t *mbar, uint32_t parity, volatile i
     }
 }
 
+__device__ __forceinline__ void arrive(uint64_t *mbar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" : : "r"(tc::smem_u32(mbar)) : "memory");
+}
+
 __device__ __forceinline__ void mma_f16(uint32_t dtmem, uint64_t ad, uint64_t bd, uint32_t idesc, int accumulate)
 {
     asm volatile(
@@ -215,38 +229,57 @@ __host__ __device__ constexpr uint32_t idesc(int M, int N, int bmn)
     return (1u << 4) | ((uint32_t)bmn << 16) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-// the MMAs of one K step: A at a (ND planes), B at b
-template <typename T>
-__device__ __forceinline__ void step(uint32_t d, uint64_t a, uint64_t b, int bmn, int accumulate)
+// the MMAs of one K step: A at a (ND planes of m8 rows, m8 a multiple of 8: the rows past them
+// that the MMA reads are the next plane's and give lanes that nothing reads), B at b.  The
+// issuing thread stays one or two MMAs ahead of the tensor cores, so what it has to wait for
+// besides (mid) goes before the last and largest MMA
+template <typename T, typename F>
+__device__ __forceinline__ void step(uint32_t d, uint64_t a, int m8, uint64_t b, int bmn, bool first, F &&mid)
 {
     constexpr int ND = Num<T>::ND, NV = Num<T>::NV;
+    if (first) {                       // digit 0 spans every group: it clears them
+        mma_f16(d, a, b, idesc(128, NV * ND, bmn), 0);
 #pragma unroll
-    for (int i = 0; i < ND; i++)
-        mma_f16(d + NV * i, a + (uint64_t)(i * (APL >> 4)), b, idesc(128, NV * (ND - i), bmn), i ? 1 : accumulate);
+        for (int i = ND - 1; i > 0; i--) {
+            if (i == 1) mid();
+            mma_f16(d + NV * i, a + (uint64_t)(i * m8 * 2), b, idesc(128, NV * (ND - i), bmn), 1);
+        }
+    } else {
+#pragma unroll
+        for (int i = ND - 1; i >= 0; i--) {
+            if (i == 0) mid();
+            mma_f16(d + NV * i, a + (uint64_t)(i * m8 * 2), b, idesc(128, NV * (ND - i), bmn), 1);
+        }
+    }
 }
 
-// eight columns of this thread's lane, without the wait
-__device__ __forceinline__ void ld8_nw(uint32_t taddr, uint32_t *r)
+template <int N> __device__ __forceinline__ void regs_up()
 {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N> __device__ __forceinline__ void regs_down()
+{
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+
+// four columns of this thread's lane, without the wait
+__device__ __forceinline__ void ld4_nw(uint32_t taddr, uint32_t *r)
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(taddr));
 }
 
-__device__ __forceinline__ void regs8(uint32_t *r)
-{
-    asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]));
-}
-
-// the accumulators of eight columns of this thread's lane, groups nv columns apart
+// the accumulators of four columns of this thread's lane, groups nv columns apart
 template <int ND>
-__device__ __forceinline__ void load_groups(uint32_t taddr, int nv, uint32_t (&v)[ND][8])
+__device__ __forceinline__ void load_groups(uint32_t taddr, int nv, uint32_t (&v)[ND][4])
 {
 #pragma unroll
-    for (int g = 0; g < ND; g++) ld8_nw(taddr + nv * g, v[g]);
+    for (int g = 0; g < ND; g++) ld4_nw(taddr + nv * g, v[g]);
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int g = 0; g < ND; g++) regs8(v[g]);
+    for (int g = 0; g < ND; g++)
+        asm volatile("" : "+r"(v[g][0]), "+r"(v[g][1]), "+r"(v[g][2]), "+r"(v[g][3]));
 }
 
 }  // namespace fx

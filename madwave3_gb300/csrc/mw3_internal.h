@@ -211,9 +211,10 @@ struct Ctx {
     // the DSTs from exact digits on the tensor cores (mw3_fx.cu): FP64, and mixed shapes outside the fused chain
     bool use_fx = false;
     int fx_grid = 0, fx_drop = 0;
+    int fx_nst[3] = {2, 2, 2};       // stages of the matrix ring: along R, along r1, angles
     void *d_fxR[2] = {nullptr, nullptr};   // digits of S2: first and second transform (__half planes)
     void *d_fxr = nullptr;           // digits of S1 of every length
-    void *d_fxe = nullptr;           // k-space factor of every length, [nn][n2] by stored column
+    void *d_fxe = nullptr;           // k-space factor of every length, [n2][nn] by stored column
     int64_t *d_fxe_off = nullptr;    // [W][na]
     void *d_fxZ = nullptr;           // second scratch rectangle, where a length exceeds 128
     void *d_fx_rows = nullptr, *d_fx_cols = nullptr;     // the tiles
