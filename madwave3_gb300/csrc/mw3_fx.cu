@@ -51,6 +51,8 @@ struct Args {
     double *H;
     const int *mapT;
     const int64_t *foff;
+    const double *psi;           // the vector itself, for the points that the transforms do not reach
+    const int *qptr, *qlist;     // per (wave, angle): stored points with r1 beyond the length
     // angular terms
     const int *map;
     const T *yj;                 // [G][na][n1] yyy(j, r1) by ladder slot
@@ -206,6 +208,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tb = *slot;
+    tc::dependents_launch();
     const int n2 = p.n2, n1 = p.n1;
     const bool vec = n2 % (32 / (int)sizeof(T)) == 0;     // rows start on 32 bytes
     auto length = [&](const Item &it) { return ANG ? p.na : ROWS ? n2 : it.nn; };
@@ -289,6 +292,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
         int ni = 0;
         Item nxt = {};
         if ((int)blockIdx.x < p.nitems) nxt = p.items[blockIdx.x];
+        tc::dependents_wait();
         for (int i = blockIdx.x; i < p.nitems; i += gridDim.x, ni++) {
             const Item it = nxt;
             if (i + (int)gridDim.x < p.nitems) nxt = p.items[i + gridDim.x];
@@ -302,6 +306,16 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
             const int k = md == 0 ? out : 2 * out + md - 1;             // the output itself
             const int pos = md == 0 ? out : p.perm && !(L & 1) ? out + (md == 1 ? 0 : L2) : k;
             const bool any = __any_sync(0xffffffffu, on);
+            if (EPI == EPI_GATHER && it.v0 == 0 && it.mode == 1) {
+                // once a segment: the stored points beyond the r1 length keep psi
+                const int wa = p.blk_wave[it.seg / p.na] * p.na + a, q1 = p.qptr[wa + 1];
+                const int64_t o = p.foff[it.seg];
+                for (int q = p.qptr[wa] + (int)threadIdx.x - FILL; q < q1; q += WAYBACK) {
+                    const int ir = p.qlist[q];
+                    p.H[o + ir] = p.psi[o + ir];
+                }
+                __syncwarp();
+            }
             const bool ok = wait(&tfull[ni & 1], (ni >> 1) & 1, fail);
             if (!__all_sync(0xffffffffu, ok)) break;
             tc::fence_after_sync();
@@ -445,10 +459,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
         int nb = 0, ni = 0;                       // B blocks written, tiles done
         bool bad = false;
         Item nxt = {};
-        if ((int)blockIdx.x < p.nitems) {
-            nxt = p.items[blockIdx.x];
-            fetch(nxt);
-        }
+        if ((int)blockIdx.x < p.nitems) nxt = p.items[blockIdx.x];
+        tc::dependents_wait();
+        if ((int)blockIdx.x < p.nitems) fetch(nxt);
         for (int i = blockIdx.x; i < p.nitems; i += gridDim.x, ni++) {
             const Item it = nxt;
             const int md = it.mode & 3, L = length(it), K = md ? (L + 1) >> 1 : L;
@@ -665,7 +678,7 @@ void set_smem()
 template <typename T, int EPI, bool FOLD>
 void launch(Ctx &c, const fx::Args<T> &p)
 {
-    fx::k_fx_dst<T, EPI, FOLD><<<std::min(p.nitems, c.fx_grid), fx::THREADS, fx::Size<T>::SMEM, c.stream>>>(p);
+    launch_early(fx::k_fx_dst<T, EPI, FOLD>, dim3(std::min(p.nitems, c.fx_grid)), fx::THREADS, fx::Size<T>::SMEM, c.stream, p);
     c.launches++;
 }
 
@@ -986,13 +999,14 @@ void launch_fx_ang(Ctx &c, const T *X, T *Y, double *H, int g_begin, int g_end)
 // the four products of the radial kinetic term of blocks [g_begin, g_end): X -> Y, Y in place
 // (or through Z), Y -> H at the stored points
 template <typename T>
-void launch_fx_dst(Ctx &c, const T *X, T *Y, double *H, int g_begin, int g_end, bool mark)
+void launch_fx_dst(Ctx &c, const T *X, T *Y, double *H, const double *psi, int g_begin, int g_end, bool mark)
 {
     const int s0 = g_begin * c.na, s1 = g_end * c.na;
     fx::Args<T> p = {};
     p.n1 = c.n1; p.n2 = c.n2; p.na = c.na;
     p.blk_wave = c.d_blk_wave;
     p.H = H; p.mapT = c.d_mapT; p.foff = c.d_foff;
+    p.psi = psi; p.qptr = c.d_quirk_ptr; p.qlist = c.d_quirk;
     p.err = c.d_tc_err;
     p.etab = (const T *)c.d_fxe; p.etoff = c.d_fxe_off;
     const fx::Item *rows = (const fx::Item *)c.d_fx_rows + c.h_fx_row0[s0];
@@ -1020,8 +1034,8 @@ void launch_fx_dst(Ctx &c, const T *X, T *Y, double *H, int g_begin, int g_end, 
     launch<T, fx::EPI_GATHER, true>(c, p);
 }
 
-template void launch_fx_dst<double>(Ctx &, const double *, double *, double *, int, int, bool);
-template void launch_fx_dst<float>(Ctx &, const float *, float *, double *, int, int, bool);
+template void launch_fx_dst<double>(Ctx &, const double *, double *, double *, const double *, int, int, bool);
+template void launch_fx_dst<float>(Ctx &, const float *, float *, double *, const double *, int, int, bool);
 template void launch_fx_ang<double>(Ctx &, const double *, double *, double *, int, int);
 template void launch_fx_ang<float>(Ctx &, const float *, float *, double *, int, int);
 

@@ -404,12 +404,12 @@ int encode_tc_dst2d_xmap(Ctx &c);
 // the [R][r1] rectangle is possible: fused split-FP16 DST and factorised angular kernel,
 // no electronic Coriolis coupling, n1 a multiple of 4 and at least 32
 bool xt_eligible(const Ctx &c);
-void launch_tc_dst2d(Ctx &c, const float *X, float *H, int g_begin, int g_end);
+void launch_tc_dst2d(Ctx &c, const float *X, float *H, const double *psi, int g_begin, int g_end);
 std::vector<double> dst_matrix(int n);
 // radial DSTs from exact digits (mw3_fx.cu); sets c.use_fx
 int build_fx(Ctx &c);
 template <typename T>
-void launch_fx_dst(Ctx &c, const T *X, T *Y, double *H, int g_begin, int g_end, bool mark);
+void launch_fx_dst(Ctx &c, const T *X, T *Y, double *H, const double *psi, int g_begin, int g_end, bool mark);
 // angular terms through the j basis, from exact digits; sets c.use_fx_ang
 int build_fx_ang(Ctx &c);
 template <typename T>

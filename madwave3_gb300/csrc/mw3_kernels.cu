@@ -20,6 +20,7 @@
 #include <mutex>
 
 #include "mw3_internal.h"
+#include "mw3_tc.cuh"
 
 namespace mw3 {
 
@@ -30,7 +31,7 @@ namespace mw3 {
 // ---------------------------------------------------------------------------
 constexpr int kPointChunk = 1024;   // stored points per CTA in the point kernels
 
-__device__ __forceinline__ float f64_to_f32_int(double x);
+using tc::f64_to_f32_int;
 template <typename T> __device__ __forceinline__ T rect_value(double v) { return (T)v; }
 // FP32 rectangles take the update kernel's rounding, so a restart reproduces a run
 template <> __device__ __forceinline__ float rect_value<float>(double v) { return f64_to_f32_int(v); }
@@ -443,24 +444,6 @@ static RaderTab rd_tab(const Ctx &c)
     return r;
 }
 
-// double -> float, round to nearest even, with integer instructions only (the
-// F2F conversion issues on the FP64 pipe); magnitudes below FLT_MIN go to a
-// signed zero, above FLT_MAX to infinity
-__device__ __forceinline__ float f64_to_f32_int(double x)
-{
-    unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    unsigned int sign = (unsigned int)(b >> 32) & 0x80000000u;
-    int e = (int)((b >> 52) & 0x7FF) - 1023 + 127;
-    if (e <= 0) return __uint_as_float(sign);
-    if (e >= 255) return __uint_as_float(sign | 0x7F800000u);
-    unsigned int m = (unsigned int)((b >> 29) & 0x7FFFFFu);
-    unsigned int rest = (unsigned int)(b & 0x1FFFFFFFu);
-    unsigned int r = ((unsigned int)e << 23) | m;
-    if (rest > 0x10000000u || (rest == 0x10000000u && (m & 1u))) r += 1u;   // carry may round into the exponent
-    if (r >= 0x7F800000u) r = 0x7F800000u;
-    return __uint_as_float(sign | r);
-}
-
 // exact float -> double with integer instructions (the F2F conversion issues
 // on the FP64 pipe); subnormal inputs become a signed zero
 __device__ __forceinline__ double f32_to_f64_int(float f)
@@ -493,7 +476,8 @@ __global__ void k_h32_to_h(DevGrid d, const float *__restrict__ h32, double *__r
     for (int ir = blockIdx.y * kPointChunk + threadIdx.x; ir < n; ir += blockDim.x) H[off + ir] = f32_to_f64_int(h32[off + ir]);
 }
 
-// stored points with ir1 beyond the DST length keep psi as their "kinetic" term
+// stored points with ir1 beyond the DST length keep psi as their "kinetic" term (the fused
+// chain and the digit transforms do it in their last kernel)
 template <typename HT>
 __global__ void k_quirk(DevGrid d, const double *__restrict__ psi, HT *__restrict__ H,
                         const int *__restrict__ qptr, const int *__restrict__ qlist, int seg0)
@@ -725,6 +709,7 @@ __device__ __forceinline__ void upd_fe(const UpdArgs &u, double *zf, int w, int6
 template <typename T, typename HT>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3) k_update(DevGrid d, UpdArgs u, T *__restrict__ X)
 {
+    tc::dependents_launch();
     const UpdChunk cd = u.desc[blockIdx.x];
     const int seg = cd.seg, chunk = cd.chunk_ns & 255, nsrc = cd.chunk_ns >> 8;
     const int a = cd.wa & 255, w = cd.wa >> 8;
@@ -1624,11 +1609,9 @@ void launch_hphi(Ctx &c, const double *psi, int g_begin, int g_end)
     if (sizeof(T) == 4 && c.use_tc_dst2d) {
         // mixed path: the whole DST chain of each slab in one tensor-core kernel, H in FP32
         stage_mark(c, 0);
-        launch_tc_dst2d(c, (const float *)c.d_X, c.d_h32, g_begin, g_end);
+        launch_tc_dst2d(c, (const float *)c.d_X, c.d_h32, psi, g_begin, g_end);
         stage_mark(c, 1);
         stage_mark(c, 2);
-        k_quirk<float><<<ng * c.na, 128, 0, c.stream>>>(d, psi, c.d_h32, c.d_quirk_ptr, c.d_quirk, g_begin * c.na);
-        LAUNCH_CHECK(c);
         stage_mark(c, 3);
         if (c.use_tc_ang) {
             launch_tc_ang(c, (const float *)c.d_X, c.d_h32, g_begin, g_end, c.x_t);
@@ -1641,7 +1624,7 @@ void launch_hphi(Ctx &c, const double *psi, int g_begin, int g_end)
         LAUNCH_CHECK(c);
     } else if (c.use_fx) {
         // the four products from exact digits on the tensor cores
-        launch_fx_dst<T>(c, (const T *)c.d_X, (T *)c.d_Y, c.d_h, g_begin, g_end, true);
+        launch_fx_dst<T>(c, (const T *)c.d_X, (T *)c.d_Y, c.d_h, psi, g_begin, g_end, true);
     } else if (sizeof(T) == 4 && tc_dst_supported(c)) {
         // mixed path: the three DST passes on the tensor cores
         launch_tc_dst(c, (const float *)c.d_X, (float *)c.d_Y, c.d_h, g_begin, g_end, 0);
@@ -1674,7 +1657,9 @@ void launch_hphi(Ctx &c, const double *psi, int g_begin, int g_end)
         LAUNCH_CHECK(c);
     }
     // points beyond the r1 DST length keep psi
-    if (!(sizeof(T) == 4 && c.use_tc_dst2d)) {
+    if (c.use_fx) {
+        stage_mark(c, 3);
+    } else if (!(sizeof(T) == 4 && c.use_tc_dst2d)) {
         k_quirk<double><<<ng * c.na, 128, 0, c.stream>>>(d, psi, c.d_h, c.d_quirk_ptr, c.d_quirk, g_begin * c.na);
         LAUNCH_CHECK(c);
         stage_mark(c, 3);
@@ -2246,7 +2231,7 @@ static void noalloc_hphi(Ctx &c, const WaveTables &t, unsigned char *scratch, co
     // the digit products, unless a folded length along r1 needs a second scratch rectangle
     const bool fx = c.use_fx && !c.d_fxZ;
     if (fx) {
-        launch_fx_dst<T>(c, X, Y, H, g0, g1, false);
+        launch_fx_dst<T>(c, X, Y, H, P, g0, g1, false);
     } else {
         if (rader)
             k_dst_rows_rader<false><<<rd_grid(), 256, 0, c.stream>>>(d, (const double *)X, (double *)Y, nullptr,
@@ -2267,8 +2252,10 @@ static void noalloc_hphi(Ctx &c, const WaveTables &t, unsigned char *scratch, co
                                                            nrows);
         LAUNCH_CHECK(c);
     }
-    k_quirk<double><<<ng * na, 128, 0, c.stream>>>(d, P, H, c.d_quirk_ptr, c.d_quirk, g0 * na);
-    LAUNCH_CHECK(c);
+    if (!fx) {
+        k_quirk<double><<<ng * na, 128, 0, c.stream>>>(d, P, H, c.d_quirk_ptr, c.d_quirk, g0 * na);
+        LAUNCH_CHECK(c);
+    }
     if (sizeof(T) == 4 && c.use_tc_ang) {
         launch_tc_ang(c, (const float *)X, H, g0, g1, false);   // its own scratch, [r1][R]
     } else if (c.use_fx_ang) {

@@ -215,5 +215,47 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
                  : "memory");
 }
 
+// programmatic dependent launch: the next kernel of the stream may start (its part before
+// dependents_wait, which reads only tables) once every CTA of this one has come here
+__device__ __forceinline__ void dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// the kernels before this one in the stream are complete and their writes visible
+__device__ __forceinline__ void dependents_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// double -> float, round to nearest even, with integer instructions only (the
+// F2F conversion issues on the FP64 pipe); magnitudes below FLT_MIN go to a
+// signed zero, above FLT_MAX to infinity
+__device__ __forceinline__ float f64_to_f32_int(double x)
+{
+    unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    unsigned int sign = (unsigned int)(b >> 32) & 0x80000000u;
+    int e = (int)((b >> 52) & 0x7FF) - 1023 + 127;
+    if (e <= 0) return __uint_as_float(sign);
+    if (e >= 255) return __uint_as_float(sign | 0x7F800000u);
+    unsigned int m = (unsigned int)((b >> 29) & 0x7FFFFFu);
+    unsigned int rest = (unsigned int)(b & 0x1FFFFFFFu);
+    unsigned int r = ((unsigned int)e << 23) | m;
+    if (rest > 0x10000000u || (rest == 0x10000000u && (m & 1u))) r += 1u;   // carry may round into the exponent
+    if (r >= 0x7F800000u) r = 0x7F800000u;
+    return __uint_as_float(sign | r);
+}
+
 }  // namespace tc
+
+// a launch whose kernel may start before the one ahead of it in the stream has ended; the
+// kernel calls tc::dependents_wait before it touches anything that one reads or writes
+template <typename... P, typename... A>
+inline void launch_early(void (*k)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
 }  // namespace mw3

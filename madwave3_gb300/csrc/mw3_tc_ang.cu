@@ -163,11 +163,20 @@ __global__ void __launch_bounds__(256, 2) k_tc_ang(AngArgs<HT> p)
     __syncthreads();
     fence_after_sync();
     const uint32_t tb = *slot;
+    dependents_launch();
     const int na = p.na, n1 = p.n1, n2 = p.n2;
     const int tile = p.tiles[blockIdx.x];
     const int r1_0 = tile >> 16, r2_0 = tile & 0xFFFF;
     const int ch = p.chain0 + blockIdx.y;
     const int cb = p.chain_ptr[ch], L = p.chain_ptr[ch + 1] - cb;
+    uint32_t ph0 = 0, ph1 = 0;
+    bool bad = false, copy_out = false;
+    // the first block's D, a table, comes with the map while the kernel ahead ends
+    if (threadIdx.x == 0 && L > 0) {
+        mbar_expect_tx(&bars[0], 2 * AG_DPLANE);
+        bulk_g2s(DS, p.dfw + (size_t)p.chain[cb] * 2 * 64 * AG_K, 2 * AG_DPLANE, &bars[0]);
+        copy_out = true;
+    }
     // the tile's map, once for the whole chain (a quarter warp reads 8 consecutive R)
     for (int e = threadIdx.x; e < AG_K * 128; e += blockDim.x) {
         int a = e >> 7, mm = e & 127;
@@ -181,8 +190,7 @@ __global__ void __launch_bounds__(256, 2) k_tc_ang(AngArgs<HT> p)
     const int ir1 = r1_0 + (m >> 3), ir2 = r2_0 + (m & 7);
     const int cr1 = min(ir1, n1 - 1), cr2 = min(ir2, n2 - 1);
     const uint32_t lrow = tb + ((uint32_t)(q4 * 32) << 16);
-    uint32_t ph0 = 0, ph1 = 0;
-    bool bad = false, copy_out = false;
+    dependents_wait();
     if (L > 0) ang_copy_x(p, p.chain[cb], r1_0, r2_0, AS + AG_APLANE);
 
     for (int pos = -1; pos < L; pos++) {
@@ -218,7 +226,7 @@ __global__ void __launch_bounds__(256, 2) k_tc_ang(AngArgs<HT> p)
         // ---- grid -> j basis for the next block of the chain, into ring slot (pos+1)%3 ----
         if (pos + 1 < L) {
             int gn = p.chain[cb + pos + 1];
-            if (threadIdx.x == 0) {
+            if (threadIdx.x == 0 && pos >= 0) {
                 mbar_expect_tx(&bars[0], 2 * AG_DPLANE);
                 bulk_g2s(DS, p.dfw + (size_t)gn * 2 * 64 * AG_K, 2 * AG_DPLANE, &bars[0]);
                 copy_out = true;
@@ -546,7 +554,7 @@ static void tc_ang_launch(Ctx &c, const float *X, HT *H, int g_begin, int g_end,
     p.na = c.na; p.n1 = c.n1; p.n2 = c.n2; p.chain0 = ch0;
     p.xt = xt ? 1 : 0;
     p.err = c.d_tc_err;
-    k_tc_ang<HT><<<dim3(c.ang_ntiles, nch), 256, smem, c.stream>>>(p);
+    launch_early(k_tc_ang<HT>, dim3(c.ang_ntiles, nch), 256, smem, c.stream, p);
     c.launches++;
 }
 

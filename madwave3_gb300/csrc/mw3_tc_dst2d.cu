@@ -55,6 +55,8 @@ constexpr uint32_t D2_BYTES = D2_NS * D2_STAGE;         // 192 KB
 constexpr int D2_NKH = 128 / D2_KC;                     // K chunks of a 128-wide operand
 constexpr size_t D2_CHUNK = D2_SMALL / 4;               // floats of one 128-row chunk (hi + lo)
 
+constexpr int D2_FILL = 16;                            // fill warps
+
 struct Dst2Args {
     const float *X;               // rectangle [G][na][n1][n2]
     float *H;                     // H psi without V, FP32
@@ -70,6 +72,8 @@ struct Dst2Args {
     int wave;                     // CTAs resident at once (one per SM): the next wave's slab is seg + wave
     const int64_t *foff;
     const int *blk_wave;
+    const double *psi;            // the vector itself: stored points beyond the r1 length keep it
+    const int *qptr, *qlist;      // per (wave, angle): those points
     int na, n1, n2, seg0;
     int *err;
 };
@@ -93,6 +97,34 @@ __device__ __forceinline__ void d2_prefetch_map(const Dst2Args &p, int a, int m,
             if (i < h) asm volatile("prefetch.global.L1 [%0];" ::"l"(mT + (size_t)i * n1 + m));
             if (i < n2 - h) asm volatile("prefetch.global.L1 [%0];" ::"l"(mT + (size_t)(n2 - 1 - i) * n1 + m));
         }
+    }
+}
+
+// the stored points with r1 beyond the transform's length keep psi: each fill thread's first
+// one is read before the products (the loads depend on one another), the others at the end
+struct D2Quirk {
+    int ir;
+    float v;
+};
+
+__device__ __forceinline__ D2Quirk d2_quirk_load(const Dst2Args &p, int wa, int64_t fo)
+{
+    D2Quirk k{-1, 0.f};
+    const int q = p.qptr[wa] + (int)threadIdx.x;
+    if (q < p.qptr[wa + 1]) {
+        k.ir = p.qlist[q];
+        k.v = f64_to_f32_int(p.psi[fo + k.ir]);
+    }
+    return k;
+}
+
+__device__ __forceinline__ void d2_quirk_store(const Dst2Args &p, int wa, int64_t fo, const D2Quirk &k)
+{
+    if (k.ir < 0) return;
+    p.H[fo + k.ir] = k.v;
+    for (int q = p.qptr[wa] + (int)threadIdx.x + D2_FILL * 32; q < p.qptr[wa + 1]; q += D2_FILL * 32) {
+        const int ir = p.qlist[q];
+        p.H[fo + ir] = f64_to_f32_int(p.psi[fo + ir]);
     }
 }
 
@@ -221,7 +253,6 @@ __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap *map, int x, i
 // parity and K chunk), with no integer division per chunk.  After any wait
 // runs out of time the CTA's shared failure flag makes every later wait return
 // at once, so a fault ends the kernel instead of hanging it.
-constexpr int D2_FILL = 16;                        // fill warps
 constexpr int D2_WARPS = D2_FILL + 2;
 constexpr int D2_MMA_WARP = D2_FILL, D2_COPY_WARP = D2_FILL + 1;
 
@@ -311,6 +342,7 @@ __global__ void __launch_bounds__(D2_WARPS * 32, 1) k_tc_dst2d(Dst2Args p, const
     __syncthreads();
     fence_after_sync();
     const uint32_t tb = *slot;
+    dependents_launch();
     const int NT = (n2 + 127) / 128;                    // R tiles of D2 and of the D3 columns
     const int RB = 128 * NT;
     const uint32_t big_lo = (uint32_t)RB * D2_KC * 4;   // lo plane of an RB-row operand
@@ -324,6 +356,7 @@ __global__ void __launch_bounds__(D2_WARPS * 32, 1) k_tc_dst2d(Dst2Args p, const
 
     if (warp == D2_COPY_WARP) {
         // ---- bulk copies of the DST-matrix operands ----
+        dependents_wait();
         if (lane == 0)
             d2_for_chunks(nkh, nkr, [&](int t, int gi, int par, int jc) {
                 if (*fail) return;
@@ -408,6 +441,8 @@ __global__ void __launch_bounds__(D2_WARPS * 32, 1) k_tc_dst2d(Dst2Args p, const
             if (p.rows_ok[a]) d2_stage_rows(p, a, s_rows, D2_FILL * 32);
             asm volatile("bar.sync 1, %0;" ::"n"(D2_FILL * 32) : "memory");
         }
+        dependents_wait();
+        const D2Quirk quirk = d2_quirk_load(p, w * na + a, p.foff[seg]);
         // second and third products: sub & 1 picks the row set, sub >> 1 the 8-column half
         const int rset = sub & 1, colh = sub >> 1;
         const int rR = 128 * rset + m;                  // the R row this thread fills in the third product
@@ -506,6 +541,7 @@ __global__ void __launch_bounds__(D2_WARPS * 32, 1) k_tc_dst2d(Dst2Args p, const
         d2_wait(&empty[(total - 1) & (D2_NS - 1)], ((total - 1) >> 2) & 1, fail);
         fence_after_sync();
         if (!*fail) d2_store_h(p, a, p.foff[seg], m, nn, h, sub, lrow, 1.f, srow);
+        d2_quirk_store(p, w * na + a, p.foff[seg], quirk);
     }
     // before shared and tensor memory are released, the async work this CTA issued
     // must be done: the copy warp waits for its last copy, the MMA warp for its
@@ -685,6 +721,7 @@ __global__ void __launch_bounds__(D2_WARPS * 32, 1) k_tc_dst2d_h(Dst2hArgs P, co
     __syncthreads();
     fence_after_sync();
     const uint32_t tb = *slot;
+    dependents_launch();
     const int NT = (n2 + 127) / 128;
     const int RB = 128 * NT;
     const uint32_t big_lo = (uint32_t)RB * H_KC * 2;    // lo plane of an RB-row operand
@@ -701,6 +738,7 @@ __global__ void __launch_bounds__(D2_WARPS * 32, 1) k_tc_dst2d_h(Dst2hArgs P, co
         // takes (one CTA per SM, issued in order) streams into L2, so that slab's first
         // product finds its tiles there instead of waiting on DRAM chunk by chunk
         const int nxt = (int)blockIdx.x + p.wave;
+        dependents_wait();
         if (lane == 0)
             h_for_chunks(nkh, nkr, [&](int t, int s, int ph, int gi, int par, int jc) {
                 if (*fail) return;
@@ -784,6 +822,14 @@ __global__ void __launch_bounds__(D2_WARPS * 32, 1) k_tc_dst2d_h(Dst2hArgs P, co
         const int m = q4 * 32 + lane;
         const uint32_t lrow = tb + ((uint32_t)(q4 * 32) << 16);
         const float divi = 1.0f / (4.0f * (float)(nn + 1) * (float)(n2 + 1));
+        {
+            const float *p1f = p.p2r1f + ((size_t)w * na + a) * n1;
+            if (threadIdx.x < 128) s_p1f[threadIdx.x] = threadIdx.x < nn ? p1f[threadIdx.x] : 0.f;
+            if (p.rows_ok[a]) d2_stage_rows(p, a, s_rows, D2_FILL * 32);
+            asm volatile("bar.sync 1, %0;" ::"n"(D2_FILL * 32) : "memory");
+        }
+        dependents_wait();
+        const D2Quirk quirk = d2_quirk_load(p, w * na + a, p.foff[seg]);
         // the slab's scales (powers of two, see above)
         const float xm = __uint_as_float(P.xmax[seg]);
         int ex = 0;
@@ -793,12 +839,6 @@ __global__ void __launch_bounds__(D2_WARPS * 32, 1) k_tc_dst2d_h(Dst2hArgs P, co
         int s_exp = sx_exp - 40;                        // sum of the operand scales' exponents (D1, D3: -20)
         constexpr float a13 = 1.f / 1048576.f;          // 2^-20
         float sc2 = 1.f;                                // D2 o F's scale, set when the second product completes
-        {
-            const float *p1f = p.p2r1f + ((size_t)w * na + a) * n1;
-            if (threadIdx.x < 128) s_p1f[threadIdx.x] = threadIdx.x < nn ? p1f[threadIdx.x] : 0.f;
-            if (p.rows_ok[a]) d2_stage_rows(p, a, s_rows, D2_FILL * 32);
-            asm volatile("bar.sync 1, %0;" ::"n"(D2_FILL * 32) : "memory");
-        }
         const int rset = sub & 1, colq = sub >> 1;
         const int rR = 128 * rset + m;
         const float e2 = (rset < NT && rR < n2) ? p.p2r2f[((size_t)w * na + a) * n2 + rR] : 0.f;
@@ -976,6 +1016,7 @@ __global__ void __launch_bounds__(D2_WARPS * 32, 1) k_tc_dst2d_h(Dst2hArgs P, co
         d2_wait(&empty[pt], pph, fail);
         fence_after_sync();
         if (!*fail) d2_store_h(p, a, p.foff[seg], m, nn, h, sub, lrow, ldexpf(1.f, -(4 * H_S_EXP + s_exp)), srow);
+        d2_quirk_store(p, w * na + a, p.foff[seg], quirk);
     }
     const int lt = total - 1, ls = lt % H_NS, lph = (lt / H_NS) & 1;
     if (lane == 0 && warp == D2_COPY_WARP && copies > 0) {
@@ -1198,7 +1239,7 @@ int encode_tc_dst2d_xmap(Ctx &c)
     return MW3_OK;
 }
 
-void launch_tc_dst2d(Ctx &c, const float *X, float *H, int g_begin, int g_end)
+void launch_tc_dst2d(Ctx &c, const float *X, float *H, const double *psi, int g_begin, int g_end)
 {
     using namespace tc;
     static bool attr = false;
@@ -1226,6 +1267,7 @@ void launch_tc_dst2d(Ctx &c, const float *X, float *H, int g_begin, int g_end)
         if (nsm <= 0) nsm = 1;
     }
     p.wave = nsm;
+    p.psi = psi; p.qptr = c.d_quirk_ptr; p.qlist = c.d_quirk;
     p.na = c.na; p.n1 = c.n1; p.n2 = c.n2; p.seg0 = g_begin * c.na;
     p.err = c.d_tc_err;
     CUtensorMap xmap;
@@ -1238,9 +1280,9 @@ void launch_tc_dst2d(Ctx &c, const float *X, float *H, int g_begin, int g_end)
         P.b.s1off = c.d_dst_s1off16;
         P.xmax = c.d_xmax;
         P.xt = c.x_t ? 1 : 0;
-        k_tc_dst2d_h<<<nseg, D2_WARPS * 32, smem, c.stream>>>(P, xmap);
+        launch_early(k_tc_dst2d_h, dim3(nseg), D2_WARPS * 32, smem, c.stream, P, xmap);
     } else {
-        k_tc_dst2d<<<nseg, D2_WARPS * 32, smem, c.stream>>>(p, xmap);
+        launch_early(k_tc_dst2d, dim3(nseg), D2_WARPS * 32, smem, c.stream, p, xmap);
     }
     c.launches++;
 }
