@@ -211,7 +211,8 @@ int build_device(Ctx &c)
         return MW3_ERR_STATE;
     }
     free_device(c);
-    c.fl_pending = c.cv_pending = false;
+    c.fl_pending = 0;
+    c.cv_pending = false;
     int na = c.na, n1 = c.n1, n2 = c.n2, ne = c.ne;
     int W = (int)c.waves.size();
     c.ang_cw = c.k_cw > 0 ? c.k_cw : c.ang_cw_fit;
@@ -890,7 +891,8 @@ int check_device_flags(Ctx &c, const char *where)
 
 int reset_accumulators(Ctx &c)
 {
-    c.fl_pending = c.cv_pending = false;
+    c.fl_pending = 0;
+    c.cv_pending = false;
     size_t nf = (size_t)std::max(c.NF, 1) * c.netot * 2;
     if (c.d_cvcring)
         MW3_CUDA_TRY(cudaMemsetAsync(c.d_cvcring, 0, sizeof(float) * mw3::kFluxRing * c.netot * 2, c.stream));
@@ -1270,7 +1272,8 @@ int mw3_run(mw3_ctx *h, int64_t n)
         for (size_t i = old; i < c.prof_ev.size(); i++) MW3_CUDA_TRY(cudaEventCreate(&c.prof_ev[i]));
         c.prof_cap = need;
     }
-    if (n > 0) c.fl_pending = c.cv_pending = true;
+    if (n > 0) c.cv_pending = true;
+    c.fl_pending += n;
     for (int64_t s = 0; s < n;) {
         if (graph_ready(c, n - s)) {
             // kGraphIters iterations as one graph replay

@@ -289,7 +289,8 @@ struct Ctx {
     float *d_cring = nullptr;        // [kFluxSlots][netot][2]
     // iterations since the rings were last added in full: without any, reading the
     // accumulators need not add the (cleared) rings again
-    bool fl_pending = false, cv_pending = false;
+    int64_t fl_pending = 0;
+    bool cv_pending = false;
     int fl_q = 32;                   // a slice of the flux points is flushed every fl_q iterations
     // mixed path: the Cvj projection in FP32 (from the FP32 copy of psi) and Cvj of the
     // last kFluxRing iterations with their C_k(E) (slot = iteration mod kFluxRing),
