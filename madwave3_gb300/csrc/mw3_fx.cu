@@ -115,6 +115,12 @@ __device__ __forceinline__ void store4(float *q, int n, bool vec, const float (&
     }
 }
 
+// the bits of a fixed-point number kept where a vector's entry was
+__device__ __forceinline__ long long as_int(double x) { return __double_as_longlong(x); }
+__device__ __forceinline__ int as_int(float x) { return __float_as_int(x); }
+__device__ __forceinline__ void as_num(long long v, double &x) { x = __longlong_as_double(v); }
+__device__ __forceinline__ void as_num(int v, float &x) { x = __int_as_float(v); }
+
 // a barrier of the filling warps; true for all of them where any of them passes true
 __device__ __forceinline__ bool barrier_or(bool x)
 {
@@ -212,6 +218,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
     const int n2 = p.n2, n1 = p.n1;
     const bool vec = n2 % (32 / (int)sizeof(T)) == 0;     // rows start on 32 bytes
     auto length = [&](const Item &it) { return ANG ? p.na : ROWS ? n2 : it.nn; };
+    // this CTA's tiles.  Along R a run of the list, where the tiles of the same vectors stand
+    // together: first the even outputs' 128-row blocks, then the odd ones'.  A second block
+    // takes the digits of the first (K is above 128 then and fills both B blocks), an odd
+    // tile what its even one has loaded
+    const int step_i = ROWS ? 1 : (int)gridDim.x;
+    const int begin = ROWS ? (int)((int64_t)p.nitems * blockIdx.x / gridDim.x) : (int)blockIdx.x;
+    const int end = ROWS ? (int)((int64_t)p.nitems * (blockIdx.x + 1) / gridDim.x) : p.nitems;
+    auto same_vectors = [](const Item &x, const Item &y) { return ROWS && x.seg == y.seg && x.v0 == y.v0; };
+    auto same_digits = [&](const Item &x, const Item &y) { return same_vectors(x, y) && ((x.mode ^ y.mode) & 3) == 0; };
     // the largest entries' exponent field of vector n of the j-th tile
     auto field = [&](int j, int n) {
         const unsigned *sx = s_max + (j % NEF) * WPG * NV;
@@ -225,7 +240,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
             // ---- the matrix steps of every tile in turn, nst in flight ----
             int ct = 0, cs = 0, cph = 0;                   // copies issued; the next one's stage and phase
             bool ok = true;
-            for (int i = blockIdx.x; i < p.nitems && ok; i += gridDim.x) {
+            for (int i = begin; i < end && ok; i += step_i) {
                 const int n = p.items[i].nks;
                 const uint32_t cb = (uint32_t)(p.items[i].nv_m8 >> 8) * (ND * 32);
                 const unsigned char *ca = p.planes + (int64_t)p.items[i].a[p.pass] * 256;
@@ -247,12 +262,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
             const uint64_t a0 = tc::sdesc(tc::smem_u32(As), LBO, SBO), b0 = tc::sdesc(tc::smem_u32(Bs), LBO, SBO);
             int t = 0, ts = 0, tph = 0;                    // steps issued; the next one's stage and phase
             int nb = 0, ni = 0;
-            bool ok = (int)blockIdx.x < p.nitems && wait(&full[0], 0, fail);
-            int nks = ok ? p.items[blockIdx.x].nks : 0, m8 = ok ? p.items[blockIdx.x].nv_m8 >> 8 : 0;
-            for (int i = blockIdx.x; i < p.nitems && ok; i += gridDim.x, ni++) {
-                const int nx = i + (int)gridDim.x;
-                const bool more = nx < p.nitems;
-                const int nks2 = more ? p.items[nx].nks : 0, m82 = more ? p.items[nx].nv_m8 >> 8 : 0;
+            bool ok = begin < end && wait(&full[0], 0, fail);
+            Item it = {}, nxt = {};
+            if (ok) it = p.items[begin];
+            for (int i = begin; i < end && ok; i += step_i, ni++) {
+                const bool more = i + step_i < end;
+                if (more) nxt = p.items[i + step_i];
+                const int nks = it.nks, m8 = it.nv_m8 >> 8;
+                const bool keep = more && same_digits(it, nxt);     // the next tile takes these B blocks again
+                const int nb0 = nb;
                 if (ni >= 2) ok = wait(&tempty[ni & 1], ((ni >> 1) - 1) & 1, fail);
                 const uint32_t d = tb + 256u * (ni & 1);
                 for (int ks = 0; ks < nks && ok; ks++) {
@@ -272,13 +290,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                             });
                     tc::mma_commit(&empty[s]);
                     if (lastk || (ks + 1) % (KB / KS) == 0) {
-                        tc::mma_commit(&bempty[nb & 1]);
+                        if (!keep) tc::mma_commit(&bempty[nb & 1]);
                         nb++;
                     }
                     if (lastk) tc::mma_commit(&tfull[ni & 1]);
                 }
-                nks = nks2;
-                m8 = m82;
+                if (keep) nb = nb0;
+                it = nxt;
             }
             // no MMA stays in flight
             for (int c = max(0, t - nst); c < t; c++) tc::mbar_wait(&empty[c % nst], (c / nst) & 1);
@@ -289,13 +307,17 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
         regs_down<REG_WAY>();
         const int q4 = warp & 3, half = (warp >> 2) & 1, m = q4 * 32 + lane;
         const uint32_t lrow = tb + ((uint32_t)(q4 * 32) << 16);
-        int ni = 0;
+        int ni = 0, nf = 0;                       // tiles done; the fill that this one's digits are from
         Item nxt = {};
-        if ((int)blockIdx.x < p.nitems) nxt = p.items[blockIdx.x];
+        if (begin < end) nxt = p.items[begin];
         tc::dependents_wait();
-        for (int i = blockIdx.x; i < p.nitems; i += gridDim.x, ni++) {
+        for (int i = begin; i < end; i += step_i, ni++) {
             const Item it = nxt;
-            if (i + (int)gridDim.x < p.nitems) nxt = p.items[i + gridDim.x];
+            bool keep = false;
+            if (i + step_i < end) {
+                nxt = p.items[i + step_i];
+                keep = same_digits(it, nxt);
+            }
             const int a = ANG ? 0 : it.seg % p.na;
             const int md = it.mode & 3, mt = it.mode >> 2;
             const int L = length(it), nv = it.nv_m8 & 255;
@@ -347,7 +369,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                     uint32_t g[ND];
 #pragma unroll
                     for (int q = 0; q < ND; q++) g[q] = v[q][c];
-                    y[c] = combine(g, field(ni, c0 + c), sh);
+                    y[c] = combine(g, field(nf, c0 + c), sh);
                 }
                 if (on) {
                     if (EPI == EPI_ROWS) {
@@ -381,6 +403,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
             tc::fence_before_sync();
             __syncwarp();
             if (lane == 0) arrive(&tempty[ni & 1]);
+            if (!keep) nf++;
         }
     } else {
         // ---- vectors into digits ----
@@ -412,10 +435,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
             }
         };
         // a tile's first B block into registers, and the largest entries past it
-        auto fetch = [&](const Item &it) {
+        auto fetch = [&](const Item &it, bool known) {
             const int L = length(it), md = it.mode & 3, K = md ? (L + 1) >> 1 : L;
             if (ROWS) {
                 const bool on = rn < (it.nv_m8 & 255);
+                if (known && K <= KB) return;
                 kmax[0] = 0;
 #pragma unroll
                 for (int u = 0; u < U; u++) {
@@ -424,7 +448,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                     for (int c = 0; c < 8; c++) kv[u][c] = kw[FOLD ? u : 0][c] = (T)0;
                     if (on && k < K) row(it, L, k, kv[u], kw[FOLD ? u : 0]);
                 }
-                if (on)
+                if (on && !known)
 #pragma unroll 1
                     for (int k = KB + 8 * rp; k < K; k += 32 * WPG) {
                         T v[8], w[8];
@@ -456,13 +480,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                 }
             }
         };
-        int nb = 0, ni = 0;                       // B blocks written, tiles done
-        bool bad = false;
+        int nb = 0, ni = 0;                       // B blocks written, tiles filled
+        bool bad = false, known = false;          // known: the tile before had the same vectors
+        unsigned mrow = 0;                        // along R: the row's largest |x|
         Item nxt = {};
-        if ((int)blockIdx.x < p.nitems) nxt = p.items[blockIdx.x];
+        if (begin < end) nxt = p.items[begin];
         tc::dependents_wait();
-        if ((int)blockIdx.x < p.nitems) fetch(nxt);
-        for (int i = blockIdx.x; i < p.nitems; i += gridDim.x, ni++) {
+        if (begin < end) fetch(nxt, false);
+        for (int i = begin, in; i < end; i = in, ni++) {
             const Item it = nxt;
             const int md = it.mode & 3, L = length(it), K = md ? (L + 1) >> 1 : L;
             const int nv = it.nv_m8 & 255;
@@ -470,14 +495,16 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
             // ---- the largest |x| of each vector ----
             unsigned *sx = s_max + (ni % NEF) * WPG * NV;
             if (ROWS) {
-                unsigned mx = kmax[0];
+                if (!known) {
+                    mrow = kmax[0];
 #pragma unroll
-                for (int u = 0; u < U; u++)
+                    for (int u = 0; u < U; u++)
 #pragma unroll
-                    for (int c = 0; c < 8; c++) mx = max(mx, max(mag(kv[u][c]), mag(kw[FOLD ? u : 0][c])));
-                mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-                mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-                if (lane < 8) sx[hf * NV + rn] = mx;
+                        for (int c = 0; c < 8; c++) mrow = max(mrow, max(mag(kv[u][c]), mag(kw[FOLD ? u : 0][c])));
+                    mrow = max(mrow, __shfl_xor_sync(0xffffffffu, mrow, 8));
+                    mrow = max(mrow, __shfl_xor_sync(0xffffffffu, mrow, 16));
+                }
+                if (lane < 8) sx[hf * NV + rn] = mrow;
             } else {
 #pragma unroll
                 for (int c = 0; c < 8; c++) {
@@ -492,7 +519,16 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                 }
             }
             if (barrier_or(bad)) break;           // every filling thread, or none
-            if (i + (int)gridDim.x < p.nitems) nxt = p.items[i + gridDim.x];
+            const bool formed = known && K <= KB;      // the differences are in the registers
+            in = i + step_i;
+            known = false;
+            for (; in < end; in += step_i) {
+                nxt = p.items[in];
+                if (!same_digits(it, nxt)) {
+                    known = same_vectors(it, nxt);
+                    break;
+                }
+            }
             // ---- digits, one block of K at a time ----
             for (int kb = 0; kb < K; kb += KB, nb++) {
                 const int kr = (min(K - kb, KB) + KS - 1) & ~(KS - 1);
@@ -517,13 +553,16 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                         Int X[8];
 #pragma unroll
                         for (int c = 0; c < 8; c++) {
-                            X[c] = 0;
-                            if (rn < nv && k + c < K) {
-                                X[c] = to_fixed(kv[u][c], ef, sh);
+                            X[c] = formed ? as_int(kv[u][c]) : 0;
+                            if (!formed && rn < nv && k + c < K) {
+                                const Int x = to_fixed(kv[u][c], ef, sh);
                                 // the middle of an odd length pairs with itself
-                                const Int Y = L - 1 - (k + c) != k + c ? to_fixed(kw[FOLD ? u : 0][7 - c], ef, sh)
-                                                                       : md == 2 ? X[c] : 0;
-                                X[c] = md == 1 ? X[c] + Y : X[c] - Y;
+                                const bool mid = L - 1 - (k + c) == k + c;
+                                const Int y = mid ? 0 : to_fixed(kw[FOLD ? u : 0][7 - c], ef, sh), z = mid ? 0 : x - y;
+                                X[c] = md == 1 ? x + y : z;
+                                if (K <= KB) as_num(z, kv[u][c]);
+                            } else if (!formed && K <= KB) {
+                                as_num((Int)0, kv[u][c]);
                             }
                         }
                         put_digits(X, Bb + (kg >> 1) * BSTEP + (rn >> 3) * SBO + (kg & 1) * LBO + (rn & 7) * 16,
@@ -557,7 +596,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                 if (lane == 0 && !bad) arrive(&bfull[nb & 1]);
             }
             bad = __any_sync(0xffffffffu, bad);
-            if (i + (int)gridDim.x < p.nitems) fetch(nxt);
+            if (in < end) fetch(nxt, known);
         }
     }
     tc::fence_before_sync();

@@ -97,3 +97,22 @@ def test_non_finite_input_stays_non_finite(shape_run):
     # subnormal and huge vectors scale as FP64 does
     assert np.allclose(p.hphi(psi * 2.0 ** 900), clean * 2.0 ** 900, rtol=1e-12)
     p.close()
+
+
+# enough tiles that a CTA takes several in a row and the later ones share the vectors, their
+# digits or their differences: odd and even R lengths, one and two B blocks and 128-row blocks,
+# runs of tiles that begin inside a group
+SHARED = [("fp64", 40, 65, 120, {}), ("fp64", 130, 257, 24, {}), ("fp64", 64, 512, 40, {}), ("fp64", 200, 96, 60, {}),
+          ("fp64", 145, 255, 20, {}), ("mixed", 150, 385, 40, {}), ("mixed", 145, 129, 90, {}), ("mixed", 256, 258, 30, {})]
+
+
+@pytest.mark.parametrize("precision,n1,n2,na,extra", SHARED)
+def test_tiles_that_share_vectors(shape_run, precision, n1, n2, na, extra):
+    run = shape_run(n1, n2, na, extra)
+    p = Propagator(run, precision)
+    psi = np.random.default_rng([n1, n2, na]).uniform(-1, 1, run.ntot)
+    h, e = p.hphi(psi), Oracle(run).hphi(psi)
+    # as the shapes with a tile a CTA
+    assert np.abs(h - e).max() <= (1e-13 if precision == "fp64" else 1e-6) * np.abs(e).max()
+    assert np.array_equal(p.hphi(psi), h)
+    p.close()
