@@ -529,7 +529,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                     break;
                 }
             }
-            // ---- digits, one block of K at a time ----
+            // ---- digits, one block of K at a time.  Every entry is converted and masked: a
+            // branch round each kept the eight chains of a thread from overlapping ----
             for (int kb = 0; kb < K; kb += KB, nb++) {
                 const int kr = (min(K - kb, KB) + KS - 1) & ~(KS - 1);
                 unsigned char *Bb = Bs + (nb & 1) * BBYTES;
@@ -551,18 +552,18 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                         const int kg = rp + 4 * WPG * u, k = kb + 8 * kg;
                         if (8 * kg >= kr) continue;
                         Int X[8];
+                        if (formed) {
 #pragma unroll
-                        for (int c = 0; c < 8; c++) {
-                            X[c] = formed ? as_int(kv[u][c]) : 0;
-                            if (!formed && rn < nv && k + c < K) {
-                                const Int x = to_fixed(kv[u][c], ef, sh);
+                            for (int c = 0; c < 8; c++) X[c] = as_int(kv[u][c]);
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < 8; c++) {
+                                const Int x = to_fixed(kv[u][c], ef, sh), y = to_fixed(kw[FOLD ? u : 0][7 - c], ef, sh);
                                 // the middle of an odd length pairs with itself
-                                const bool mid = L - 1 - (k + c) == k + c;
-                                const Int y = mid ? 0 : to_fixed(kw[FOLD ? u : 0][7 - c], ef, sh), z = mid ? 0 : x - y;
-                                X[c] = md == 1 ? x + y : z;
+                                const Int on = -(Int)(rn < nv && k + c < K), two = -(Int)(L - 1 - (k + c) != k + c);
+                                const Int z = (x - y) & on & two;
+                                X[c] = md == 1 ? (x + (y & two)) & on : z;
                                 if (K <= KB) as_num(z, kv[u][c]);
-                            } else if (!formed && K <= KB) {
-                                as_num((Int)0, kv[u][c]);
                             }
                         }
                         put_digits(X, Bb + (kg >> 1) * BSTEP + (rn >> 3) * SBO + (kg & 1) * LBO + (rn & 7) * 16,
@@ -577,14 +578,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
 #pragma unroll
                         for (int c = 0; c < 8; c++) {
                             const int ef = field(ni, 8 * grp + c);
-                            X[c] = 0;
-                            if (k < K) {
-                                X[c] = to_fixed(kv[u][c], ef, sh);
-                                if (FOLD && md) {
-                                    const Int Y =
-                                        L - 1 - k != k ? to_fixed(kw[FOLD ? u : 0][c], ef, sh) : md == 2 ? X[c] : 0;
-                                    X[c] = md == 1 ? X[c] + Y : X[c] - Y;
-                                }
+                            const Int on = -(Int)(k < K);
+                            X[c] = to_fixed(kv[u][c], ef, sh) & on;
+                            if (FOLD) {
+                                // a length kept whole pairs with nothing, an odd one's middle with itself
+                                const Int y = to_fixed(kw[FOLD ? u : 0][c], ef, sh) & on;
+                                const Int two = -(Int)(L - 1 - k != k);
+                                X[c] = md == 2 ? (X[c] - y) & two : X[c] + (y & two & -(Int)(md == 1));
                             }
                         }
                         put_digits(X, Bb + (kl >> 4) * BSTEP + grp * SBO + ((kl >> 3) & 1) * LBO + (kl & 7) * 16,
