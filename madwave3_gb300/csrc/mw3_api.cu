@@ -215,6 +215,9 @@ int build_device(Ctx &c)
     c.cv_pending = false;
     int na = c.na, n1 = c.n1, n2 = c.n2, ne = c.ne;
     int W = (int)c.waves.size();
+    int64_t points = 0;
+    for (auto &t : c.waves) points += t.ntot;
+    c.acc_beside = points <= (int64_t)1 << 26;
     c.ang_cw = c.k_cw > 0 ? c.k_cw : c.ang_cw_fit;
     // ---- shared grid ----
     TRY(dupload(c, &c.d_indr1, c.indr1));
@@ -1154,13 +1157,17 @@ void join_acc(Ctx &c)
 
 // one Chebyshev iteration of every wave: H psi and the update on the context's stream, the
 // accumulators beside the next iteration's H psi (in sequence while stages are timed).  One
-// J = 0 wave leaves most SMs idle in both, and their launches add up: 78 us an iteration in
-// sequence, of which the accumulators 35
+// J = 0 wave leaves most SMs idle in both, and their launches add up: mixed 256 x 128 x 60
+// took 78 us an iteration in sequence, of which the accumulators 35; beside each other 66,
+// and 53 with the programmatic launches of the H psi kernels.  Above 2^26 stored points in
+// sequence again: H psi fills the chip and loses more to the accumulators beside it than
+// they take alone.  In sequence against beside, us an iteration, mixed 256 x 128 x 60: 51.3 M
+// points 2399, 2287; 73.4 M 3342, 3350; 88.0 M 3985, 4011; 147 M 6545, 6680
 void run_iteration(Ctx &c)
 {
     int64_t it = c.it + 1;
     const int par = (int)(it & 1);
-    const bool beside = c.side && !c.prof;
+    const bool beside = c.side && !c.prof && c.acc_beside;
     hphi_all(c, c.d_pk, 0, c.G);
     if (c.nofemax > 0) mw3::launch_fe_coef(c, it);
     // psi_it overwrites psi_it-2 and its norm partials: its accumulators must be through

@@ -289,6 +289,7 @@ struct Ctx {
     float *d_cring = nullptr;        // [kFluxSlots][netot][2]
     // iterations since the rings were last added in full: without any, reading the
     // accumulators need not add the (cleared) rings again
+    bool acc_beside = false;         // accumulators beside the next H psi (see run_iteration)
     int64_t fl_pending = 0;
     bool cv_pending = false;
     int fl_q = 32;                   // a slice of the flux points is flushed every fl_q iterations
