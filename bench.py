@@ -225,13 +225,13 @@ def dominant_roofline(stages, nrec, model, kin, precision, nsto, peaks):
              "r1 pair: 4 nopr1^2 npun2; explicit angular: 2 nangu per stored point, the l^2 stage for up "
              "to three coupled blocks)")
     if kind == "flop" and precision == "fp64":
-        # the FP64 path's transforms run on the FP64 pipe: against its nominal rate
-        # (the measured peaks hold no FP64 figure)
+        # FP64 results, so against the FP64 pipe's nominal rate (the measured peaks hold no
+        # FP64 figure); products from exact digits on the tensor cores can pass it
         achieved = work / t_launch / 1e12
         return {"bound": "fp64", "achieved": achieved, "peak": FP64_NOMINAL_TFLOPS, "unit": "TFLOP/s",
                 "frac": achieved / FP64_NOMINAL_TFLOPS, "traffic": traffic, "kernel": dom,
                 "peak_source": "nominal GB300 FP64 rate (not measured)",
-                "work": flops % ", run as a Rader FFT with fewer flops when npun2 = 256"}
+                "work": flops % ", formed from exact digits on the tensor cores for npun2 <= 512"}
     if kind == "flop" and not on_tensor:
         achieved = work / t_launch / 1e12
         return {"bound": "fp32", "achieved": achieved, "peak": FP32_NOMINAL_TFLOPS, "unit": "TFLOP/s",

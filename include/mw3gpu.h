@@ -208,7 +208,9 @@ int mw3_set_ecoriolis(mw3_ctx *ctx, int32_t wave_id, int32_t on);
  * single CPU code path has none).  choice[4]:
  *   [0] radial DST form -- mixed: 0 fused split-FP16 tcgen05 chain, 1 fused
  *       3xTF32 chain, 2 three-kernel tensor-core DST, 3 CUDA-core FP32 DST;
- *       FP64: 0 folded dense DST-I, 1 Rader FFT along R (npun2 = 256);
+ *       FP64: 0 folded dense DST-I, 1 Rader FFT along R (npun2 = 256), both on
+ *       CUDA cores; the built-in rule runs exact digit products on the tensor
+ *       cores for npun2 <= 512 (no flag of mw3_path_flags stands for those);
  *   [1] FP32 rectangle stored [R][r1]: 0 no, 1 yes (where eligible);
  *   [2] mixed angular terms: 0 explicit kernels, 1 factorised tensor-core kernel;
  *   [3] R-column chunk of the explicit angular kernels: 8..64, a power of two;
@@ -249,7 +251,7 @@ int mw3_kernel_launches(mw3_ctx *ctx, int64_t *count);
 #define MW3_PATH_TC_DST_FUSED 4   /* the whole radial DST chain in one kernel per (block, angle) */
 #define MW3_PATH_DST_F16 8        /* the fused chain as split-FP16 products (MW3_DST_TF32=1 selects 3xTF32) */
 #define MW3_PATH_X_T 16           /* the FP32 rectangle stored [R][r1] (MW3_X_T=1; default [r1][R]) */
-#define MW3_PATH_RADER 32         /* FP64: the DST along R by Rader's FFT (npun2 = 256) */
+#define MW3_PATH_RADER 32         /* FP64: the DST along R by Rader's FFT (npun2 = 256, when pinned) */
 int mw3_path_flags(mw3_ctx *ctx, int32_t *flags);
 
 /* The CUDA stream (cudaStream_t) all device work of the context runs on, for

@@ -172,7 +172,9 @@ __device__ __forceinline__ void ang_values(const Args<T> &p, int g, int j, int r
 // With every warp of a CTA going through these phases in turn, two CTAs an SM, a tile of 32
 // FP64 vectors took 40 k cycles a CTA: 5 k for the loads, 7 k for the digits, 11 k for the
 // MMAs, 7-20 k for the way back.  The MMAs of a K step take 500 cycles; with the copies and
-// their waits on the issuing thread it was 1400.
+// their waits on the issuing thread it was 1400.  Cycles a tile now (FP64, 384 x 192 x 80):
+// along R 14 k, the MMAs; along r1 13-16 k, fill and way back 10 k each beside them; to the j
+// basis 10 k, back 12 k, of which the loads of the coupled blocks 9 k.
 template <typename T, int EPI, bool FOLD>
 __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
 {
@@ -221,7 +223,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
     // this CTA's tiles.  Along R a run of the list, where the tiles of the same vectors stand
     // together: first the even outputs' 128-row blocks, then the odd ones'.  A second block
     // takes the digits of the first (K is above 128 then and fills both B blocks), an odd
-    // tile what its even one has loaded
+    // tile what its even one has loaded.  With a fill for every tile that was 22 k cycles at
+    // K = 192, against 10-14 k for the MMAs (mixed 384 x 192 x 80, first transform: 623 us,
+    // sharing 419).  Along r1 (K up to 128, one row block) runs of tiles gained nothing in
+    // FP32 (740 -> 738 us) and lost in FP64 (1248 -> 1354): strided there
     const int step_i = ROWS ? 1 : (int)gridDim.x;
     const int begin = ROWS ? (int)((int64_t)p.nitems * blockIdx.x / gridDim.x) : (int)blockIdx.x;
     const int end = ROWS ? (int)((int64_t)p.nitems * (blockIdx.x + 1) / gridDim.x) : p.nitems;
@@ -996,10 +1001,10 @@ int build_fx_ang_t(Ctx &c)
 }  // namespace
 
 // tables of the digit DSTs; leaves c.use_fx false where another path is asked for or the shape
-// is outside them.  Mixed: the fused chain is faster (one kernel, 2.6 against an estimated 4 ms
-// on the J = 0..40 sweep), and the three-kernel 3xTF32 form keeps its shapes (every r1 length up
+// is outside them.  Mixed: the fused chain is faster (256 x 128 x 60, J = 10: 141 us against 449),
+// and the three-kernel 3xTF32 form keeps its shapes (every r1 length up
 // to 128): results there would otherwise move by its own error, 2e-5 of psi after 32 iterations
-// at npun2 = 436; what is left ran on FP32 CUDA cores (512 x 256 x 120: 1.56 ms against 0.74)
+// at npun2 = 436; what is left ran on FP32 CUDA cores (512 x 256 x 120: 1.56 ms against 0.47)
 int build_fx(Ctx &c)
 {
     c.use_fx = false;

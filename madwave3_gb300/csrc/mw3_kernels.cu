@@ -6,11 +6,15 @@
 //   2. k_dst_cols   S1 (E o (S1 Y))                (DST-I along r twice, k-space scaling between)
 //   3. k_dst_rows   Y x S2 with a gather epilogue  (kinetic part at the stored points)
 //      k_quirk      stored points with ir1 > nopr1 keep psi (the reference's DST never
-//                   reaches them, mod_Hphi_01y2.f:768-831)
+//                   reaches them, mod_Hphi_01y2.f:768-831); the fused and the digit
+//                   DST write those points themselves
 //   4. k_ang_j      j^2 part: per r1, dense angle x angle matrix (xj2)
 //      k_ang_l      l^2 part incl. Omega+-1 Coriolis coupling: per R (xl2p)
 //   5. k_update     V psi, damped three-term recursion, next rectangle, norm partials
-// followed by the accumulators (CoefEcheby, totalflux_k, Cvjflux_k).
+// Stages 1-4 are these kernels only where neither the fused tensor-core kernels
+// (mw3_tc_dst2d.cu, mw3_tc_ang.cu) nor the exact-digit ones (mw3_fx.cu) apply: FP64
+// beyond npun2 = 512 or 256 angles, pinned choices, the entry point without allocation.
+// Then the accumulators (CoefEcheby, totalflux_k, Cvjflux_k).
 // T is the transform type: double (plain FP64 path) or float (mixed path); the
 // recursion vectors, potential, absorption and accumulators are always FP64.
 #include <math.h>
