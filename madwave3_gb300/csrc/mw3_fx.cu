@@ -232,10 +232,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
     const int end = ROWS ? (int)((int64_t)p.nitems * (blockIdx.x + 1) / gridDim.x) : p.nitems;
     auto same_vectors = [](const Item &x, const Item &y) { return ROWS && x.seg == y.seg && x.v0 == y.v0; };
     auto same_digits = [&](const Item &x, const Item &y) { return same_vectors(x, y) && ((x.mode ^ y.mode) & 3) == 0; };
-    // the largest entries' exponent field of vector n of the j-th tile
+    // the largest entries' exponent field of vector n of the j-th tile; a vector of subnormal
+    // numbers has the scale of the smallest normal ones, which is theirs
     auto field = [&](int j, int n) {
         const unsigned *sx = s_max + (j % NEF) * WPG * NV;
-        return (int)((WPG == 2 ? max(sx[n], sx[NV + n]) : sx[n]) >> Num<T>::EBITS);
+        return max((int)((WPG == 2 ? max(sx[n], sx[NV + n]) : sx[n]) >> Num<T>::EBITS), 1);
     };
 
     constexpr int MMA_WARP = (FILL + WAYBACK) / 32;
