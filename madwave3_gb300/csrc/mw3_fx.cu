@@ -58,7 +58,10 @@ struct Args {
     const T *yj;                 // [G][na][n1] yyy(j, r1) by ladder slot
     const T *l2;                 // [G][3][na][n2] xl2mat_j(Om, Om + q; R), slot q + 1, by ladder slot
     const int *cpl;              // [G][3][2]: the block Omega + q of the same wave and state, -1 where there is none
-    int dexp;                    // the angular matrices' scale 2^dexp
+    // [G][na] each angle's scale: its entries of the angular matrices stand x 2^sa, the vector's over it.
+    // Next to the poles every entry of a high Omega is tiny (60 angles, Omega = 10: 2e-13), and with one
+    // scale for the whole matrix it kept what it has of the 54 bits: 9e-9 of its own size there
+    const int *sa;
     int *err;
 };
 
@@ -232,11 +235,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
     const int end = ROWS ? (int)((int64_t)p.nitems * (blockIdx.x + 1) / gridDim.x) : p.nitems;
     auto same_vectors = [](const Item &x, const Item &y) { return ROWS && x.seg == y.seg && x.v0 == y.v0; };
     auto same_digits = [&](const Item &x, const Item &y) { return same_vectors(x, y) && ((x.mode ^ y.mode) & 3) == 0; };
-    // the largest entries' exponent field of vector n of the j-th tile; a vector of subnormal
-    // numbers has the scale of the smallest normal ones, which is theirs
+    // the largest entries' exponent field of vector n of the j-th tile
     auto field = [&](int j, int n) {
         const unsigned *sx = s_max + (j % NEF) * WPG * NV;
-        return max((int)((WPG == 2 ? max(sx[n], sx[NV + n]) : sx[n]) >> Num<T>::EBITS), 1);
+        return (int)((WPG == 2 ? max(sx[n], sx[NV + n]) : sx[n]) >> Num<T>::EBITS);
     };
 
     constexpr int MMA_WARP = (FILL + WAYBACK) / 32;
@@ -327,10 +329,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
             const int a = ANG ? 0 : it.seg % p.na;
             const int md = it.mode & 3, mt = it.mode >> 2;
             const int L = length(it), nv = it.nv_m8 & 255;
-            const int sh = Num<T>::SH - (md ? 1 : 0) - p.drop + (ANG ? p.dexp : 0);
             const int L2 = (L + 1) >> 1;                                // even outputs
             const int out = 128 * mt + m;                               // index within its parity
             const bool on = md == 0 ? out < L : out < (md == 1 ? L2 : L - L2);
+            const int sh = Num<T>::SH - (md ? 1 : 0) - p.drop;
+            const auto ls = lane_scale(EPI == EPI_ANG_G && on ? p.sa[(size_t)it.seg * p.na + out] : 0, (T)0);
             const int k = md == 0 ? out : 2 * out + md - 1;             // the output itself
             const int pos = md == 0 ? out : p.perm && !(L & 1) ? out + (md == 1 ? 0 : L2) : k;
             const bool any = __any_sync(0xffffffffu, on);
@@ -375,7 +378,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                     uint32_t g[ND];
 #pragma unroll
                     for (int q = 0; q < ND; q++) g[q] = v[q][c];
-                    y[c] = combine(g, field(nf, c0 + c), sh);
+                    y[c] = combine(g, field(nf, c0 + c), sh, ls);
                 }
                 if (on) {
                     if (EPI == EPI_ROWS) {
@@ -418,6 +421,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
         const int rn = (lane & 7) + 8 * grp, rp = (lane >> 3) + 4 * hf;      // along R: this thread's row and k group
         T kv[U][8], kw[FOLD ? U : 1][8];                      // entries of the first B block, and their mirrors
         unsigned kmax[ROWS ? 1 : 8];                          // the largest |x| past the first block
+        int ka[EPI == EPI_ANG_J ? U : 1];                     // the scales of kv's angles
         // entry k of this thread's eight vectors (transforms along r1, angles)
         auto column = [&](const Item &it, int k, T (&v)[8]) {
             const int n = (it.nv_m8 & 255) - 8 * grp;
@@ -427,6 +431,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                 load8(p.src + (((size_t)it.seg * p.na + k) * n1 + it.nn) * n2 + it.v0 + 8 * grp, n, vec, v);
             else
                 load8(p.src + ((size_t)it.seg * n1 + k) * n2 + it.v0 + 8 * grp, n, vec, v);
+        };
+        auto scale = [&](const Item &it, int k) { return EPI == EPI_ANG_J ? p.sa[(size_t)it.seg * p.na + k] : 0; };
+        auto scaled = [&](T x, int u) {
+            return EPI == EPI_ANG_J ? mag_down<T>(mag(x), ka[EPI == EPI_ANG_J ? u : 0]) : mag(x);
         };
         // along R: entries k..k+7 of this thread's row, and their mirrors L-1-k downwards
         auto row = [&](const Item &it, int L, int k, T (&v)[8], T (&w)[8]) {
@@ -470,6 +478,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                     const int k = lane + 32 * hf + KT * u;
 #pragma unroll
                     for (int c = 0; c < 8; c++) kv[u][c] = (T)0;
+                    if (EPI == EPI_ANG_J) ka[EPI == EPI_ANG_J ? u : 0] = k < K ? scale(it, k) : 0;
                     if (k < K) column(it, k, kv[u]);
                     if (FOLD) {
 #pragma unroll
@@ -481,8 +490,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                 for (int k = lane + 32 * hf + KB; k < K; k += KT) {
                     T v[8];
                     column(it, k, v);
+                    const int s = scale(it, k);
 #pragma unroll
-                    for (int c = 0; c < 8; c++) kmax[ROWS ? 0 : c] = max(kmax[ROWS ? 0 : c], mag(v[c]));
+                    for (int c = 0; c < 8; c++)
+                        kmax[ROWS ? 0 : c] = max(kmax[ROWS ? 0 : c], EPI == EPI_ANG_J ? mag_down<T>(mag(v[c]), s) : mag(v[c]));
                 }
             }
         };
@@ -498,7 +509,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
             const int md = it.mode & 3, L = length(it), K = md ? (L + 1) >> 1 : L;
             const int nv = it.nv_m8 & 255;
             const int sh = Num<T>::SH - (md ? 1 : 0) - p.drop;
-            // ---- the largest |x| of each vector ----
+            // ---- the largest |x| of each vector.  One of subnormal numbers has the scale of the
+            // smallest normal ones, which is theirs ----
             unsigned *sx = s_max + (ni % NEF) * WPG * NV;
             if (ROWS) {
                 if (!known) {
@@ -510,18 +522,18 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                     mrow = max(mrow, __shfl_xor_sync(0xffffffffu, mrow, 8));
                     mrow = max(mrow, __shfl_xor_sync(0xffffffffu, mrow, 16));
                 }
-                if (lane < 8) sx[hf * NV + rn] = mrow;
+                if (lane < 8) sx[hf * NV + rn] = max(mrow, 1u << Num<T>::EBITS);
             } else {
 #pragma unroll
                 for (int c = 0; c < 8; c++) {
                     unsigned mx = kmax[ROWS ? 0 : c];
 #pragma unroll
                     for (int u = 0; u < U; u++) {
-                        mx = max(mx, mag(kv[u][c]));
+                        mx = max(mx, scaled(kv[u][c], u));
                         if (FOLD) mx = max(mx, mag(kw[FOLD ? u : 0][c]));
                     }
                     mx = __reduce_max_sync(0xffffffffu, mx);
-                    if (lane == c) sx[hf * NV + 8 * grp + c] = mx;
+                    if (lane == c) sx[hf * NV + 8 * grp + c] = max(mx, 1u << Num<T>::EBITS);
                 }
             }
             if (barrier_or(bad)) break;           // every filling thread, or none
@@ -547,6 +559,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                     for (int u = 0; u < U; u++) {
                         const int k = ROWS ? kb + 8 * (rp + 4 * WPG * u) : kb + lane + 32 * hf + KT * u;
                         if (k >= K) continue;
+                        if (EPI == EPI_ANG_J) ka[EPI == EPI_ANG_J ? u : 0] = scale(it, k);
                         if (!ROWS) column(it, k, kv[u]);
                         else if (rn < nv) row(it, L, k, kv[u], kw[FOLD ? u : 0]);
                     }
@@ -583,7 +596,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                         Int X[8];
 #pragma unroll
                         for (int c = 0; c < 8; c++) {
-                            const int ef = field(ni, 8 * grp + c);
+                            const int ef = field(ni, 8 * grp + c) + (EPI == EPI_ANG_J ? ka[EPI == EPI_ANG_J ? u : 0] : 0);
                             const Int on = -(Int)(k < K);
                             X[c] = to_fixed(kv[u][c], ef, sh) & on;
                             if (FOLD) {
@@ -890,16 +903,11 @@ int build_fx_ang_t(Ctx &c)
     const int na = c.na, n1 = c.n1, n2 = c.n2, G = c.G, ne = c.ne;
     const int nks = (na + fx::KS - 1) / fx::KS, nmt = (na + 127) / 128, m8 = plane_rows(na);
     const int units = nks * step_units<T>(m8);
-    double dmax = 0.0;
     for (auto &t : c.waves)
-        for (double d : t.djmmp) {
+        for (double d : t.djmmp)
             if (!(fabs(d) <= 2.0)) return MW3_OK;
-            dmax = std::max(dmax, fabs(d));
-        }
-    int ex = 0;
-    if (dmax > 0.0) frexp(dmax, &ex);                 // dmax < 2^ex
-    const int dexp = std::min(8, std::max(0, 1 - ex));    // the largest entry just below 2
     std::vector<__half> pl;
+    std::vector<int> sa((size_t)G * na), sd(na);
     std::vector<const double *> seen;                 // the (Omega, state) columns already cut
     std::vector<int> seen_at, seen_lad;
     std::vector<T> yj((size_t)G * na * n1, (T)0), l2((size_t)G * 3 * na * n2, (T)0);
@@ -916,6 +924,15 @@ int build_fx_ang_t(Ctx &c)
             const int g = t.g0 + b, om = t.iombas[b], e = t.nelebas[b];
             const double *D = t.djmmp.data() + ((size_t)om * ne + (e - 1)) * (t.nangu2 + 1) * na;
             const int lad = (t.j0 * 4 + t.inc) * 4096 + njl;
+            // an angle's largest entry of the ladder just below 2
+            for (int a = 0; a < na; a++) {
+                double dmax = 0.0;
+                for (int js = 0; js < njl; js++) dmax = std::max(dmax, fabs(D[(size_t)(t.j0 + js * t.inc) * na + a]));
+                int ex = 1;
+                if (dmax > 0.0) frexp(dmax, &ex);         // dmax < 2^ex
+                sd[a] = std::min((int)fx::Num<T>::SAMAX, std::max(0, 1 - ex));
+            }
+            std::copy(sd.begin(), sd.end(), sa.begin() + (size_t)g * na);
             int f = -1;
             for (size_t i = 0; i < seen.size() && f < 0; i++)
                 if (seen_lad[i] == lad && !memcmp(seen[i], D, sizeof(double) * (t.nangu2 + 1) * na)) f = (int)i;
@@ -925,7 +942,7 @@ int build_fx_ang_t(Ctx &c)
                 seen_lad.push_back(lad);
                 seen_at.push_back((int)(pl.size() / 128));
                 auto d = [&](int js, int a) {
-                    return js < njl ? llrint(ldexp(D[(size_t)(t.j0 + js * t.inc) * na + a], dexp + fx::Num<T>::SBITS))
+                    return js < njl ? llrint(ldexp(D[(size_t)(t.j0 + js * t.inc) * na + a], sd[a] + fx::Num<T>::SBITS))
                                     : 0LL;
                 };
                 drop = std::max(drop, append_planes<T>(pl, na, m8, na, [&](int m, int k) { return d(m, k); }));
@@ -982,6 +999,7 @@ int build_fx_ang_t(Ctx &c)
     fx::Item *di = nullptr;
     if ((rc = fx_upload(c, &d, pl))) return rc;
     if ((rc = fx_upload(c, &di, items))) return rc;
+    if ((rc = fx_upload(c, &c.d_fx_sa, sa))) return rc;
     T *dy = nullptr, *dl = nullptr;
     if ((rc = fx_upload(c, &dy, yj))) return rc;
     if ((rc = fx_upload(c, &dl, l2))) return rc;
@@ -991,7 +1009,6 @@ int build_fx_ang_t(Ctx &c)
     c.d_fxD = d;
     c.fx_nst[2] = ring_stages<T>(m8);
     c.fx_drop_ang = drop;
-    c.fx_dexp = dexp;
     set_smem<T, fx::EPI_ANG_J, false>();
     set_smem<T, fx::EPI_ANG_G, false>();
     c.fx_grid = fx_ctas();
@@ -1032,7 +1049,7 @@ void launch_fx_ang(Ctx &c, const T *X, T *Y, double *H, int g_begin, int g_end)
     p.err = c.d_tc_err;
     p.planes = (const unsigned char *)c.d_fxD;
     p.yj = (const T *)c.d_fx_yj; p.l2 = (const T *)c.d_fx_l2; p.cpl = c.d_cpl;
-    p.drop = c.fx_drop_ang; p.dexp = c.fx_dexp; p.nst = c.fx_nst[2];
+    p.drop = c.fx_drop_ang; p.sa = c.d_fx_sa; p.nst = c.fx_nst[2];
     p.items = (const fx::Item *)c.d_fx_ang + c.h_fx_ang0[g_begin];
     p.nitems = c.h_fx_ang0[g_end] - c.h_fx_ang0[g_begin];
     p.src = X; p.dst = Y; p.pass = 0;

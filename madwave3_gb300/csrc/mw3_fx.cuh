@@ -36,11 +36,11 @@ constexpr int NEF = 8;                             // tiles whose exponents are 
 // groups of one tile take up to 256 tensor-memory columns, half of them.
 template <typename T> struct Num;
 template <> struct Num<double> {
-    enum { ND = 7, NV = 32, SH = 4, EBITS = 20, EMAX = 0x7FF, SBITS = 54 };
+    enum { ND = 7, NV = 32, SH = 4, EBITS = 20, EMAX = 0x7FF, SBITS = 54, SAMAX = 1000 };
     typedef long long Int;
 };
 template <> struct Num<float> {
-    enum { ND = 4, NV = 64, SH = 6, EBITS = 23, EMAX = 0xFF, SBITS = 29 };
+    enum { ND = 4, NV = 64, SH = 6, EBITS = 23, EMAX = 0xFF, SBITS = 29, SAMAX = 80 };
     typedef int Int;
 };
 template <typename T> struct Size {
@@ -61,8 +61,15 @@ __host__ __device__ constexpr uint32_t a_off(int r, int k)
 __device__ __forceinline__ unsigned mag(double x) { return (unsigned)__double2hiint(x) & 0x7FFFFFFFu; }
 __device__ __forceinline__ unsigned mag(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }
 
+// mag of x / 2^s (as far as its exponent field); infinities and NaN stay
+template <typename T>
+__device__ __forceinline__ unsigned mag_down(unsigned m, int s)
+{
+    return m >> Num<T>::EBITS >= (unsigned)Num<T>::EMAX ? m : (unsigned)max((int)m - (s << Num<T>::EBITS), 0);
+}
+
 // round(x 2^(57 - E)) for |x| < 2^E, E = ef - 1022 with ef the exponent field of the
-// largest |x| of the vector; sh = 4, or 3 to leave a bit for a sum of two
+// largest |x| of the vector; sh = 4, or 3 to leave a bit for a sum of two; x / 2^s with s added to ef
 __device__ __forceinline__ long long to_fixed(double x, int ef, int sh)
 {
     const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
@@ -145,10 +152,16 @@ __device__ __forceinline__ void put_digits(const int *X, unsigned char *dst, uin
     }
 }
 
+// what combine takes a row's power of two s back with: the exponent, or the factor 2^-s (s up to
+// 80, and f below is 2^-24 at least or 0, so nothing is lost)
+__device__ __forceinline__ int lane_scale(int s, double) { return s; }
+__device__ __forceinline__ float lane_scale(int s, float) { return __uint_as_float((unsigned)(127 - s) << 23); }
+
 // one output: its seven groups -> the sum over k of S x.  ef: exponent field of the vector's
-// largest |x|, sh as in to_fixed.  (Conversions by FP32 additions and integer instructions
+// largest |x|, sh as in to_fixed, ls: the power of two that this output's row of S stands
+// multiplied with (lane_scale).  (Conversions by FP32 additions and integer instructions
 // instead of the quarter-rate and FP64 units were no faster.)
-__device__ __forceinline__ double combine(const uint32_t (&v)[7], int ef, int sh)
+__device__ __forceinline__ double combine(const uint32_t (&v)[7], int ef, int sh, int ls)
 {
     int a[7];
 #pragma unroll
@@ -161,7 +174,7 @@ __device__ __forceinline__ double combine(const uint32_t (&v)[7], int ef, int sh
     if (ef >= 0x7FF) return __longlong_as_double(0x7FF8000000000000ll);   // an infinity or NaN in the vector
     if (V == 0) return 0.0;
     const double y = (double)V;
-    const int sc = ef - 1061 + (4 - sh) - z;         // E - 39 - z, one more for a folded vector
+    const int sc = ef - 1061 + (4 - sh) - z - ls;    // E - 39 - z, one more for a folded vector
     const int e = (int)(((unsigned)__double2hiint(y) >> 20) & 0x7FFu) + sc;
     if (e > 0 && e < 0x7FF)
         return __hiloint2double(__double2hiint(y) + (sc << 20), __double2loint(y));
@@ -169,11 +182,11 @@ __device__ __forceinline__ double combine(const uint32_t (&v)[7], int ef, int sh
 }
 
 // the groups are exact; their FP32 sum rounds once at the size of the first
-__device__ __forceinline__ float combine(const uint32_t (&v)[4], int ef, int sh)
+__device__ __forceinline__ float combine(const uint32_t (&v)[4], int ef, int sh, float ls)
 {
     const float r = 1.f / 256.f;
-    const float f = fmaf(fmaf(fmaf(__uint_as_float(v[3]), r, __uint_as_float(v[2])), r, __uint_as_float(v[1])), r,
-                         __uint_as_float(v[0]));
+    const float f = ls * fmaf(fmaf(fmaf(__uint_as_float(v[3]), r, __uint_as_float(v[2])), r, __uint_as_float(v[1])), r,
+                              __uint_as_float(v[0]));
     if (ef >= 0xFF) return __uint_as_float(0x7FC00000u);
     const int sc = ef - 137 + (6 - sh);              // E - 11 (48 - 29 - 30), one more for a folded vector
     const int s0 = max(sc, -100);

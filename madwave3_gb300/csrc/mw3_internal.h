@@ -221,8 +221,9 @@ struct Ctx {
     std::vector<int> h_fx_row0, h_fx_col0;               // [G na + 1] first tile of each segment
     // the angular terms through the j basis, from exact digits: FP64, and mixed above 64 angles
     bool use_fx_ang = false;
-    int fx_drop_ang = 0, fx_dexp = 0;
-    void *d_fxD = nullptr;           // digits of Djmmp, both directions, per distinct (Omega, state)
+    int fx_drop_ang = 0;
+    void *d_fxD = nullptr;           // digits of Djmmp, both directions, per distinct (Omega, state), angles scaled
+    int *d_fx_sa = nullptr;          // [G][na] by 2^sa
     void *d_fx_yj = nullptr, *d_fx_l2 = nullptr;         // [G][na][n1], [G][3][na][n2] by ladder slot
     void *d_fx_ang = nullptr;        // the tiles
     std::vector<int> h_fx_ang0;                          // [G + 1] first tile of each block

@@ -1,10 +1,12 @@
-"""The digit products at the small end: vectors of subnormal numbers."""
+"""The digit products at the small end: vectors of subnormal numbers, and the components next to
+the poles of the angular terms."""
 import os
 
 import numpy as np
 import pytest
 
 from madwave3_gb300 import Propagator
+from oracle.mw3ref import Oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -15,8 +17,8 @@ def shape_run(tmp_path_factory):
 
     def make(n1, n2, na, extra):
         d = str(tmp_path_factory.mktemp("fxs") / "case")
-        generator.write_case(d, npun1=n1, npun2=n2, nangu=na, jmax=min(na - 1, 12) // 2 * 2, nvmax=1, netot=32, npun1min=8,
-                             alpha0_bohr=1.2, **extra)
+        generator.write_case(d, **{**dict(npun1=n1, npun2=n2, nangu=na, jmax=min(na - 1, 12) // 2 * 2, nvmax=1, netot=32,
+                                          npun1min=8, alpha0_bohr=1.2), **extra})
         return setup.load(os.path.join(d, "input.dat"))
     return make
 
@@ -43,4 +45,40 @@ def test_subnormal_vectors(shape_run, precision, n1, n2, na, tiny, scale, rel):
         tol = np.ldexp(4 * n1 * n2 * (1 + run.radcutmax) / 2, tiny)
     assert tol < 2.0 ** -6 * np.abs(clean).max()
     assert np.abs(p.hphi(psi) - clean).max() <= tol + rel * np.abs(clean).max()
+    p.close()
+
+
+@pytest.mark.parametrize("precision,na,om0,om", [("fp64", 40, 9, 12), ("fp64", 130, 15, 16), ("mixed", 70, 13, 15),
+                                                 ("mixed", 130, 15, 16)])
+def test_angles_next_to_the_poles(shape_run, precision, na, om0, om):
+    """Single components of the angular terms where the associated Legendre functions are tiny (1e-8 to 1e-12
+    of their largest), for packets of a few j and for a single grid point, at one (r1, R)."""
+    run = shape_run(24, 40, na, dict(Jtot=om, iommin=om0, iommax=om, iomref=om0, jref=om0, jmax=om0))
+    p, ref = Propagator(run, precision), Oracle(run)
+    at = [{(int(x), int(y)): k for k, (x, y) in enumerate(zip(run.indr1[a, :n], run.indr2[a, :n]))}
+          for a, n in enumerate(run.npunreal)]
+    point = sorted(set.intersection(*(set(m) for m in at)))[0]
+    where = np.array([[run.offs[a, b] + at[a][point] for a in range(na)] for b in range(run.ncan)])
+    D = [run.djmmp[run.iombas[b], 0] for b in range(run.ncan)]               # [j][angle]
+    dmax = [np.abs(d).max(0) for d in D]
+    rng = np.random.default_rng([na, om])
+    top = run.ncan - 1
+    assert run.iombas[top] == om and dmax[top][0] < 1e-7
+    packets = []
+    for b in (top, 0):
+        js = [j for j in range(run.iombas[b], run.iombas[b] + 7) if j < na]
+        packets.append((b, None, D[b][js].T @ rng.normal(size=len(js))))
+        for a in (0, 1, na // 2):
+            packets.append((b, a, np.where(np.arange(na) == a, rng.normal(), 0.0)))
+    for b, only, x in packets:
+        psi = np.zeros(run.ntot)
+        psi[where[b]] = x
+        h, e = p.hphi(psi), ref.hphi(psi)
+        for t in range(max(0, b - 1), min(run.ncan, b + 2)):
+            got, want = h[where[t]], e[where[t]]
+            keep = np.arange(na) != (only if t == b else -1)                 # (its own angle has the radial terms)
+            # an angle's value is a sum over j of entries of at most dmax: na products, each way
+            size = (np.abs(want) / dmax[t])[keep].max()
+            tol = 64 * na * (2.0 ** -52 if precision == "fp64" else 2.0 ** -23) * size * dmax[t]
+            assert np.all(np.abs(got - want)[keep] <= tol[keep])
     p.close()
