@@ -210,7 +210,7 @@ int mw3_set_ecoriolis(mw3_ctx *ctx, int32_t wave_id, int32_t on);
  *       3xTF32 chain, 2 three-kernel tensor-core DST, 3 CUDA-core FP32 DST;
  *       FP64: 0 folded dense DST-I, 1 Rader FFT along R (npun2 = 256), both on
  *       CUDA cores; the built-in rule runs exact digit products on the tensor
- *       cores for npun2 <= 512 (no flag of mw3_path_flags stands for those);
+ *       cores for npun2 <= 512 (MW3_PATH_DIGIT_DST);
  *   [1] FP32 rectangle stored [R][r1]: 0 no, 1 yes (where eligible);
  *   [2] mixed angular terms: 0 explicit kernels, 1 factorised tensor-core kernel;
  *   [3] R-column chunk of the explicit angular kernels: 8..64, a power of two;
@@ -244,14 +244,18 @@ int mw3_kernel_launches(mw3_ctx *ctx, int64_t *count);
  * DSTs run on the tensor cores (with MW3_PATH_TC_DST_FUSED when as one fused
  * kernel, and MW3_PATH_DST_F16 when that kernel takes split-FP16 products
  * rather than 3xTF32), MW3_PATH_TC_ANG when the angular terms run as the
- * factorised tensor-core contraction (all mixed precision only).  No
- * reference counterpart: the reference has a single code path. */
+ * factorised tensor-core contraction (all mixed precision only);
+ * MW3_PATH_DIGIT_DST and MW3_PATH_DIGIT_ANG when they run as exact digit
+ * products on the tensor cores (both precisions).  No reference counterpart:
+ * the reference has a single code path. */
 #define MW3_PATH_TC_DST 1
 #define MW3_PATH_TC_ANG 2
 #define MW3_PATH_TC_DST_FUSED 4   /* the whole radial DST chain in one kernel per (block, angle) */
 #define MW3_PATH_DST_F16 8        /* the fused chain as split-FP16 products (MW3_DST_TF32=1 selects 3xTF32) */
 #define MW3_PATH_X_T 16           /* the FP32 rectangle stored [R][r1] (MW3_X_T=1; default [r1][R]) */
 #define MW3_PATH_RADER 32         /* FP64: the DST along R by Rader's FFT (npun2 = 256, when pinned) */
+#define MW3_PATH_DIGIT_DST 64     /* the radial DSTs from exact base-256 digits */
+#define MW3_PATH_DIGIT_ANG 128    /* the angular terms from exact base-256 digits */
 int mw3_path_flags(mw3_ctx *ctx, int32_t *flags);
 
 /* The CUDA stream (cudaStream_t) all device work of the context runs on, for

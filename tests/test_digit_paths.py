@@ -1,0 +1,67 @@
+"""Which kernels a context chooses, on the CPU: the library's host code over a stand-in CUDA
+runtime (fake_cudart.cpp) that counts device memory and launches nothing."""
+import ctypes as ct
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from madwave3_gb300 import Propagator, build, propagator
+from tests.test_gpu_fx_dst import MIXED, SHAPES, SHARED
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    gxx = shutil.which("g++")
+    if not gxx:
+        pytest.skip("no host compiler")
+    build.build()
+    objs = [os.path.join(build.OUT, s.replace(".cu", ".o")) for s in build.SOURCES]
+    if not all(os.path.exists(o) for o in objs):
+        build.build(force=True)
+    lib = str(tmp_path_factory.mktemp("fake") / "libmw3fake.so")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(build._nvcc()))), "include") \
+        if os.path.isabs(build._nvcc()) else "/usr/local/cuda/include"
+    subprocess.run([gxx, "-O1", "-std=c++17", "-fPIC", "-shared", "-I" + cuda, os.path.join(HERE, "fake_cudart.cpp")] + objs +
+                   ["-o", lib, "-Wl,-z,defs", "-lpthread", "-ldl"], check=True)
+    mp = pytest.MonkeyPatch()
+    mp.setattr(propagator, "_lib", None)
+    mp.setattr(propagator, "library_path", lambda: lib)
+    L = propagator.load_library()
+    L.fake_budget.argtypes = [ct.c_size_t]
+    L.fake_used.restype = L.fake_peak.restype = ct.c_size_t
+    yield L
+    mp.undo()
+
+
+@pytest.fixture(scope="module")
+def shape_run(tmp_path_factory):
+    from madwave3_gb300.host import generator, setup
+
+    def make(n1, n2, na, extra):
+        d = str(tmp_path_factory.mktemp("paths") / "case")
+        generator.write_case(d, npun1=n1, npun2=n2, nangu=na, jmax=min(na - 1, 12) // 2 * 2, nvmax=1, netot=32, npun1min=8,
+                             alpha0_bohr=1.2, **extra)
+        return setup.load(os.path.join(d, "input.dat"))
+    return make
+
+
+@pytest.mark.parametrize("precision,n1,n2,na,extra", [("fp64",) + s for s in SHAPES] +
+                         [("mixed",) + s for s in MIXED] + SHARED)
+def test_shapes_of_the_digit_products_take_them(fake, shape_run, precision, n1, n2, na, extra):
+    run = shape_run(n1, n2, na, extra)
+    p = Propagator(run, precision)
+    p.start()
+    path = p.path()
+    assert path["digit_dst"]
+    assert path["digit_angular"] == (precision == "fp64" or na > 64)
+    p.close()
+    p = Propagator(run, precision)
+    p.set_choices({"dst": 3 if precision == "mixed" else 0, "angular": 0})
+    p.start()
+    path = p.path()
+    assert not path["digit_dst"] and not path["digit_angular"]
+    p.close()
