@@ -18,12 +18,35 @@ using mw3::WaveTables;
 namespace {
 
 
+void drop_graphs(Ctx &c)
+{
+    for (int p = 0; p < 2; p++) {
+        if (c.graph_exec[p]) cudaGraphExecDestroy(c.graph_exec[p]);
+        c.graph_exec[p] = nullptr;
+        c.graph_launches[p] = 0;
+    }
+}
+
+// The digit transforms keep their tables, and a second rectangle where an r1 length is above
+// 128, only while there is room: an allocation that finds none has them, and the dense
+// transforms run from there on.  True if there is something more to allocate from now.
+bool give_back_digits(Ctx &c)
+{
+    if (!c.use_fx) return false;
+    cudaGetLastError();
+    if (cudaStreamSynchronize(c.stream) != cudaSuccess) return false;
+    drop_graphs(c);                  // they replay the digit kernels
+    mw3::drop_fx(c);
+    return true;
+}
+
 template <typename V>
 int dupload(Ctx &c, V **dst, const V *src, size_t n)
 {
     *dst = nullptr;
     size_t bytes = sizeof(V) * std::max<size_t>(n, 1);
     cudaError_t e = cudaMalloc((void **)dst, bytes);
+    if (e == cudaErrorMemoryAllocation && give_back_digits(c)) e = cudaMalloc((void **)dst, bytes);
     if (e != cudaSuccess) {
         c.err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
         return MW3_ERR_NOMEM;
@@ -62,14 +85,12 @@ int dalloc(Ctx &c, V **dst, size_t n, bool zero = true)
 
 void free_device(Ctx &c)
 {
-    for (int p = 0; p < 2; p++) {
-        if (c.graph_exec[p]) cudaGraphExecDestroy(c.graph_exec[p]);
-        c.graph_exec[p] = nullptr;
-        c.graph_launches[p] = 0;
-    }
+    drop_graphs(c);
     c.d_itbase = nullptr;
     for (void *p : c.allocs) cudaFree(p);
     c.allocs.clear();
+    c.fx_allocs.clear();
+    c.use_fx = c.use_fx_ang = false;
     c.built = false;
 }
 
@@ -753,8 +774,8 @@ int build_device(Ctx &c)
     mw3::set_kernel_attributes(c);
     TRY(mw3::build_tc_ang(c));
     TRY(mw3::build_tc_dst2d(c));
+    TRY(mw3::build_fx_ang(c));       // smaller than the explicit matrices, so ahead of what can be given back
     TRY(mw3::build_fx(c));
-    TRY(mw3::build_fx_ang(c));
     c.h32 = c.use_tc_dst2d && c.use_tc_ang;
     c.d_h32 = nullptr;
     c.d_vr32 = nullptr;
@@ -1419,7 +1440,10 @@ int mw3_totalflux(mw3_ctx *h, int32_t w, double *tot, double *elec)
     mw3::flush_flux(c);
     mw3::flush_cvj(c);
     const size_t row = (size_t)t.netot * (1 + c.ne);        // P(E), then each state's
-    MW3_CUDA_TRY(cudaMallocAsync(&d, sizeof(double) * row * (1 + mw3::totalflux_chunks(c, w)), c.stream));
+    const size_t bytes = sizeof(double) * row * (1 + mw3::totalflux_chunks(c, w));
+    cudaError_t e = cudaMallocAsync(&d, bytes, c.stream);
+    if (e == cudaErrorMemoryAllocation && give_back_digits(c)) e = cudaMallocAsync(&d, bytes, c.stream);
+    MW3_CUDA_TRY(e);
     mw3::launch_totalflux(c, w, d + row, d);
     MW3_CUDA_TRY(cudaMemcpyAsync(tot, d, sizeof(double) * t.netot, cudaMemcpyDeviceToHost, c.stream));
     if (elec)

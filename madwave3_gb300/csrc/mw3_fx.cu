@@ -836,8 +836,9 @@ int build_fx_t(Ctx &c)
             void *z = nullptr;
             const size_t bytes = sizeof(T) * (size_t)c.G * na * n1 * n2;
             if (cudaMalloc(&z, bytes) != cudaSuccess) {
-                cudaGetLastError();              // no room: the dense transforms need none
-                return MW3_OK;
+                cudaGetLastError();
+                c.err = "cudaMalloc: second rectangle of the digit transforms";
+                return MW3_ERR_NOMEM;
             }
             c.allocs.push_back(z);
             MW3_CUDA_TRY(cudaMemset(z, 0, bytes));
@@ -1027,15 +1028,39 @@ int build_fx(Ctx &c)
 {
     c.use_fx = false;
     c.d_fxZ = nullptr;
+    c.fx_allocs.clear();
     if (c.k_dst >= 0 || (!c.fp64 && (c.use_tc_dst2d || tc_dst_supported(c)))) return MW3_OK;
-    return c.fp64 ? build_fx_t<double>(c) : build_fx_t<float>(c);
+    const size_t n0 = c.allocs.size();
+    const int rc = c.fp64 ? build_fx_t<double>(c) : build_fx_t<float>(c);
+    c.fx_allocs.assign(c.allocs.begin() + (long)n0, c.allocs.end());
+    if (!c.use_fx) drop_fx(c);
+    return rc == MW3_ERR_NOMEM ? MW3_OK : rc;        // no room: the dense transforms need none of this
+}
+
+void drop_fx(Ctx &c)
+{
+    for (void *p : c.fx_allocs) {
+        cudaFree(p);
+        c.allocs.erase(std::find(c.allocs.begin(), c.allocs.end(), p));
+    }
+    c.fx_allocs.clear();
+    c.d_fxR[0] = c.d_fxR[1] = c.d_fxr = c.d_fxe = c.d_fxZ = c.d_fx_rows = c.d_fx_cols = nullptr;
+    c.d_fxe_off = nullptr;
+    c.use_fx = false;
 }
 
 int build_fx_ang(Ctx &c)
 {
     c.use_fx_ang = false;
     if (c.k_ang == 0 || c.na < 2 || c.na > 256 || c.use_tc_ang) return MW3_OK;
-    return c.fp64 ? build_fx_ang_t<double>(c) : build_fx_ang_t<float>(c);
+    const size_t n0 = c.allocs.size();
+    const int rc = c.fp64 ? build_fx_ang_t<double>(c) : build_fx_ang_t<float>(c);
+    if (!c.use_fx_ang)
+        while (c.allocs.size() > n0) {
+            cudaFree(c.allocs.back());
+            c.allocs.pop_back();
+        }
+    return rc == MW3_ERR_NOMEM ? MW3_OK : rc;
 }
 
 // j^2, l^2 and the Omega coupling of blocks [g_begin, g_end) (whole waves): X -> B in Y, then H +=

@@ -219,6 +219,7 @@ struct Ctx {
     void *d_fxZ = nullptr;           // second scratch rectangle, where a length exceeds 128
     void *d_fx_rows = nullptr, *d_fx_cols = nullptr;     // the tiles
     std::vector<int> h_fx_row0, h_fx_col0;               // [G na + 1] first tile of each segment
+    std::vector<void *> fx_allocs;   // all of these, given back where another allocation finds no room
     // the angular terms through the j basis, from exact digits: FP64, and mixed above 64 angles
     bool use_fx_ang = false;
     int fx_drop_ang = 0;
@@ -411,6 +412,8 @@ void launch_tc_dst2d(Ctx &c, const float *X, float *H, const double *psi, int g_
 std::vector<double> dst_matrix(int n);
 // radial DSTs from exact digits (mw3_fx.cu); sets c.use_fx
 int build_fx(Ctx &c);
+// frees their tables and clears c.use_fx
+void drop_fx(Ctx &c);
 template <typename T>
 void launch_fx_dst(Ctx &c, const T *X, T *Y, double *H, const double *psi, int g_begin, int g_end, bool mark);
 // angular terms through the j basis, from exact digits; sets c.use_fx_ang

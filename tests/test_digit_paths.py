@@ -65,3 +65,51 @@ def test_shapes_of_the_digit_products_take_them(fake, shape_run, precision, n1, 
     path = p.path()
     assert not path["digit_dst"] and not path["digit_angular"]
     p.close()
+
+
+def _context(fake, run, precision, choices=None, budget=1 << 40):
+    """(a context after a start, one H psi and one iteration; its path) under a device-memory budget."""
+    fake.fake_budget(fake.fake_used() + budget)
+    fake.fake_peak()
+    p = Propagator(run, precision)
+    if choices:
+        p.set_choices(choices)
+    p.start()
+    p.hphi(run.psi0)
+    p.run(1)
+    return p, p.path()
+
+
+# r1 lengths above 128 take a second rectangle; the last one has explicit angular matrices beside it
+@pytest.mark.parametrize("precision,n1,n2,na", [("fp64", 150, 64, 3), ("mixed", 150, 150, 3), ("mixed", 145, 69, 70),
+                                                ("fp64", 48, 127, 3)])
+def test_digit_tables_never_cost_a_context_its_memory(fake, shape_run, precision, n1, n2, na):
+    run = shape_run(n1, n2, na, {})
+    base = fake.fake_used()
+    p, path = _context(fake, run, precision)
+    assert path["digit_dst"]
+    with_digits = fake.fake_used() - base
+    p.close()
+    assert fake.fake_used() == base
+    p, path = _context(fake, run, precision, {"dst": 3 if precision == "mixed" else 0})
+    assert not path["digit_dst"]
+    dense = fake.fake_peak() - base
+    p.close()
+    assert dense < with_digits
+    # whatever the room between the two: the context works, without the digit tables
+    for k in range(17):
+        budget = dense + (with_digits - 1 - dense) * k // 16
+        p, path = _context(fake, run, precision, budget=budget)
+        assert not path["digit_dst"], budget
+        assert fake.fake_used() - base <= dense
+        p.close()
+        assert fake.fake_used() == base
+    p, path = _context(fake, run, precision, budget=with_digits)
+    assert path["digit_dst"]
+    # a later allocation that finds no room has them back
+    p.cvj_history(64)
+    p.run(1)
+    assert not p.path()["digit_dst"]
+    p.close()
+    assert fake.fake_used() == base
+    fake.fake_budget(1 << 40)
