@@ -26,7 +26,7 @@ def fake(tmp_path_factory):
     cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(build._nvcc()))), "include") \
         if os.path.isabs(build._nvcc()) else "/usr/local/cuda/include"
     subprocess.run([gxx, "-O1", "-std=c++17", "-fPIC", "-shared", "-I" + cuda, os.path.join(HERE, "fake_cudart.cpp")] + objs +
-                   ["-o", lib, "-Wl,-z,defs", "-lpthread", "-ldl"], check=True)
+                   ["-o", lib, "-Wl,-z,defs", "-Wl,-Bsymbolic", "-lpthread", "-ldl"], check=True)
     mp = pytest.MonkeyPatch()
     mp.setattr(propagator, "_lib", None)
     mp.setattr(propagator, "library_path", lambda: lib)
