@@ -727,10 +727,17 @@ int fx_upload(Ctx &c, V **dst, const std::vector<V> &v)
     return MW3_OK;
 }
 
+// the kernel's shared memory granted, and compiled with the registers that its warps share out
 template <typename T, int EPI, bool FOLD>
-void set_smem()
+bool ready()
 {
-    cudaFuncSetAttribute(fx::k_fx_dst<T, EPI, FOLD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fx::Size<T>::SMEM);
+    cudaFuncAttributes a;
+    const bool ok = cudaFuncSetAttribute(fx::k_fx_dst<T, EPI, FOLD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)fx::Size<T>::SMEM) == cudaSuccess &&
+                    cudaFuncGetAttributes(&a, fx::k_fx_dst<T, EPI, FOLD>) == cudaSuccess &&
+                    a.numRegs * fx::THREADS >= fx::REGS;
+    if (!ok) cudaGetLastError();
+    return ok;
 }
 
 template <typename T, int EPI, bool FOLD>
@@ -748,6 +755,9 @@ int build_fx_t(Ctx &c)
     c.d_fxZ = nullptr;
     // K of one product is at most 256: npun2 <= 512 folded, npun1 <= 256 (which mw3_create asks for)
     if (c.n2 > 512 || c.n1 > 256) return MW3_OK;
+    if (!(ready<T, fx::EPI_ROWS, true>() && ready<T, fx::EPI_GATHER, true>() && ready<T, fx::EPI_COLS_E, false>() &&
+          ready<T, fx::EPI_COLS, false>() && ready<T, fx::EPI_COLS_E, true>() && ready<T, fx::EPI_COLS, true>()))
+        return MW3_OK;
     const int n1 = c.n1, n2 = c.n2, na = c.na, W = (int)c.waves.size();
     int dropR = 0, drop1 = 0;
     // along R: [pass][parity][128-row block][K step]
@@ -882,12 +892,6 @@ int build_fx_t(Ctx &c)
     c.d_fx_rows = d;
     if ((rc = fx_upload(c, &d, cols))) return rc;
     c.d_fx_cols = d;
-    set_smem<T, fx::EPI_ROWS, true>();
-    set_smem<T, fx::EPI_GATHER, true>();
-    set_smem<T, fx::EPI_COLS_E, false>();
-    set_smem<T, fx::EPI_COLS, false>();
-    set_smem<T, fx::EPI_COLS_E, true>();
-    set_smem<T, fx::EPI_COLS, true>();
     c.fx_grid = fx_ctas();
     c.use_fx = true;
     return MW3_OK;
@@ -904,6 +908,7 @@ int build_fx_ang_t(Ctx &c)
     const int na = c.na, n1 = c.n1, n2 = c.n2, G = c.G, ne = c.ne;
     const int nks = (na + fx::KS - 1) / fx::KS, nmt = (na + 127) / 128, m8 = plane_rows(na);
     const int units = nks * step_units<T>(m8);
+    if (!(ready<T, fx::EPI_ANG_J, false>() && ready<T, fx::EPI_ANG_G, false>())) return MW3_OK;
     for (auto &t : c.waves)
         for (double d : t.djmmp)
             if (!(fabs(d) <= 2.0)) return MW3_OK;
@@ -1010,8 +1015,6 @@ int build_fx_ang_t(Ctx &c)
     c.d_fxD = d;
     c.fx_nst[2] = ring_stages<T>(m8);
     c.fx_drop_ang = drop;
-    set_smem<T, fx::EPI_ANG_J, false>();
-    set_smem<T, fx::EPI_ANG_G, false>();
     c.fx_grid = fx_ctas();
     c.use_fx_ang = true;
     return MW3_OK;

@@ -28,7 +28,10 @@ constexpr int THREADS = FILL + WAYBACK + 128;      // and one warp for the MMAs,
 // registers a thread: 96 at launch (640 threads), then shared out by warpgroup: 256 x 128 +
 // 256 x 80 + 128 x 64 = 61440, all that the CTA was launched with
 constexpr int REG_FILL = 128, REG_WAY = 80, REG_AUX = 64;
-static_assert(FILL * REG_FILL + WAYBACK * REG_WAY + 128 * REG_AUX <= THREADS * 96, "more registers than at launch");
+// (with fewer at launch the filling warps would wait for theirs without end: the host asks
+// the compiled kernel before it takes it)
+constexpr int REGS = FILL * REG_FILL + WAYBACK * REG_WAY + 128 * REG_AUX;
+static_assert(REGS <= THREADS * 96, "more registers than at launch");
 constexpr int NEF = 8;                             // tiles whose exponents are kept (up to five are under way)
 
 // What depends on the type of the vectors.  FP32 vectors take four digits of 30 bits

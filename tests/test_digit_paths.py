@@ -113,3 +113,19 @@ def test_digit_tables_never_cost_a_context_its_memory(fake, shape_run, precision
     p.close()
     assert fake.fake_used() == base
     fake.fake_budget(1 << 40)
+
+
+# the kernel's warps share out the registers that a CTA is launched with, 96 a thread
+@pytest.mark.parametrize("precision,n1,n2,na", [("fp64", 24, 40, 4), ("mixed", 145, 69, 70)])
+def test_a_kernel_with_fewer_registers_is_left_alone(fake, shape_run, precision, n1, n2, na):
+    run = shape_run(n1, n2, na, {})
+    try:
+        for regs, taken in ((96, True), (88, False), (102, True)):
+            fake.fake_registers(regs)
+            p = Propagator(run, precision)
+            p.start()
+            path = p.path()
+            assert path["digit_dst"] == path["digit_angular"] == taken
+            p.close()
+    finally:
+        fake.fake_registers(96)
