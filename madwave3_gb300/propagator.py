@@ -473,13 +473,22 @@ class Propagator:
 
     def path(self):
         """Kernels in use (after start): tensor-core radial DSTs, fused into one
-        kernel per slab or not (as split-FP16 or 3xTF32 products), the
-        tensor-core angular contraction, and the exact digit products of both."""
+        kernel per slab or not (as split-FP16 or 3xTF32 products), and the
+        tensor-core angular contraction."""
+        f = self._path_flags()
+        return {"tc_dst": bool(f & 1), "tc_dst_fused": bool(f & 4), "tc_angular": bool(f & 2),
+                "dst_f16": bool(f & 8), "x_transposed": bool(f & 16), "rader": bool(f & 32)}
+
+    def digit_products(self):
+        """Whether the radial DSTs and the angular terms run as exact digit
+        products on the tensor cores (after start)."""
+        f = self._path_flags()
+        return {"dst": bool(f & 64), "angular": bool(f & 128)}
+
+    def _path_flags(self):
         f = ct.c_int32()
         self._check(self.L.mw3_path_flags(self.h, ct.byref(f)), "mw3_path_flags")
-        return {"tc_dst": bool(f.value & 1), "tc_dst_fused": bool(f.value & 4), "tc_angular": bool(f.value & 2),
-                "dst_f16": bool(f.value & 8), "x_transposed": bool(f.value & 16), "rader": bool(f.value & 32),
-                "digit_dst": bool(f.value & 64), "digit_angular": bool(f.value & 128)}
+        return f.value
 
     def stream(self):
         """cudaStream_t of the context, as an integer handle."""

@@ -55,20 +55,20 @@ def test_shapes_of_the_digit_products_take_them(fake, shape_run, precision, n1, 
     run = shape_run(n1, n2, na, extra)
     p = Propagator(run, precision)
     p.start()
-    path = p.path()
-    assert path["digit_dst"]
-    assert path["digit_angular"] == (precision == "fp64" or na > 64)
+    digits = p.digit_products()
+    assert digits["dst"]
+    assert digits["angular"] == (precision == "fp64" or na > 64)
     p.close()
     p = Propagator(run, precision)
     p.set_choices({"dst": 3 if precision == "mixed" else 0, "angular": 0})
     p.start()
-    path = p.path()
-    assert not path["digit_dst"] and not path["digit_angular"]
+    digits = p.digit_products()
+    assert not digits["dst"] and not digits["angular"]
     p.close()
 
 
 def _context(fake, run, precision, choices=None, budget=1 << 40):
-    """(a context after a start, one H psi and one iteration; its path) under a device-memory budget."""
+    """(a context after a start, one H psi and one iteration; its digit products) under a device-memory budget."""
     fake.fake_budget(fake.fake_used() + budget)
     fake.fake_peak()
     p = Propagator(run, precision)
@@ -77,7 +77,7 @@ def _context(fake, run, precision, choices=None, budget=1 << 40):
     p.start()
     p.hphi(run.psi0)
     p.run(1)
-    return p, p.path()
+    return p, p.digit_products()
 
 
 # r1 lengths above 128 take a second rectangle; the last one has explicit angular matrices beside it
@@ -86,30 +86,30 @@ def _context(fake, run, precision, choices=None, budget=1 << 40):
 def test_digit_tables_never_cost_a_context_its_memory(fake, shape_run, precision, n1, n2, na):
     run = shape_run(n1, n2, na, {})
     base = fake.fake_used()
-    p, path = _context(fake, run, precision)
-    assert path["digit_dst"]
+    p, digits = _context(fake, run, precision)
+    assert digits["dst"]
     with_digits = fake.fake_used() - base
     p.close()
     assert fake.fake_used() == base
-    p, path = _context(fake, run, precision, {"dst": 3 if precision == "mixed" else 0})
-    assert not path["digit_dst"]
+    p, digits = _context(fake, run, precision, {"dst": 3 if precision == "mixed" else 0})
+    assert not digits["dst"]
     dense = fake.fake_peak() - base
     p.close()
     assert dense < with_digits
     # whatever the room between the two: the context works, without the digit tables
     for k in range(17):
         budget = dense + (with_digits - 1 - dense) * k // 16
-        p, path = _context(fake, run, precision, budget=budget)
-        assert not path["digit_dst"], budget
+        p, digits = _context(fake, run, precision, budget=budget)
+        assert not digits["dst"], budget
         assert fake.fake_used() - base <= dense
         p.close()
         assert fake.fake_used() == base
-    p, path = _context(fake, run, precision, budget=with_digits)
-    assert path["digit_dst"]
+    p, digits = _context(fake, run, precision, budget=with_digits)
+    assert digits["dst"]
     # a later allocation that finds no room has them back
     p.cvj_history(64)
     p.run(1)
-    assert not p.path()["digit_dst"]
+    assert not p.digit_products()["dst"]
     p.close()
     assert fake.fake_used() == base
     fake.fake_budget(1 << 40)
@@ -124,8 +124,8 @@ def test_a_kernel_with_fewer_registers_is_left_alone(fake, shape_run, precision,
             fake.fake_registers(regs)
             p = Propagator(run, precision)
             p.start()
-            path = p.path()
-            assert path["digit_dst"] == path["digit_angular"] == taken
+            digits = p.digit_products()
+            assert digits["dst"] == digits["angular"] == taken
             p.close()
     finally:
         fake.fake_registers(96)

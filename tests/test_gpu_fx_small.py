@@ -44,7 +44,7 @@ def test_subnormal_vectors(shape_run, precision, n1, n2, na, tiny, scale, rel):
     else:
         tol = np.ldexp(4 * n1 * n2 * (1 + run.radcutmax) / 2, tiny)
     assert tol < 2.0 ** -6 * np.abs(clean).max()
-    assert p.path()["digit_dst"]
+    assert p.digit_products()["dst"]
     assert np.abs(p.hphi(psi) - clean).max() <= tol + rel * np.abs(clean).max()
     p.close()
 
@@ -82,5 +82,5 @@ def test_angles_next_to_the_poles(shape_run, precision, na, om0, om):
             size = (np.abs(want) / dmax[t])[keep].max()
             tol = 64 * na * (2.0 ** -52 if precision == "fp64" else 2.0 ** -23) * size * dmax[t]
             assert np.all(np.abs(got - want)[keep] <= tol[keep])
-    assert p.path()["digit_angular"]
+    assert p.digit_products()["angular"]
     p.close()
