@@ -253,6 +253,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
                 const uint32_t cb = (uint32_t)(p.items[i].nv_m8 >> 8) * (ND * 32);
                 const unsigned char *ca = p.planes + (int64_t)p.items[i].a[p.pass] * 256;
                 for (int ks = 0; ks < n; ks++) {
+                    if (ct == nst) tc::dependents_wait();      // the waits have a limit, the kernel ahead has none
                     if (ct >= nst && !(ok = wait(&empty[cs], cph ^ 1, fail))) break;
                     tc::mbar_expect_tx(&full[cs], cb);
                     tc::bulk_g2s(As + cs * astage, ca + (int64_t)ks * cb, cb, &full[cs]);
@@ -270,6 +271,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fx_dst(Args<T> p)
             const uint64_t a0 = tc::sdesc(tc::smem_u32(As), LBO, SBO), b0 = tc::sdesc(tc::smem_u32(Bs), LBO, SBO);
             int t = 0, ts = 0, tph = 0;                    // steps issued; the next one's stage and phase
             int nb = 0, ni = 0;
+            tc::dependents_wait();                         // as the copies
             bool ok = begin < end && wait(&full[0], 0, fail);
             Item it = {}, nxt = {};
             if (ok) it = p.items[begin];

@@ -377,6 +377,7 @@ __global__ void __launch_bounds__(D2_WARPS * 32, 1) k_tc_dst2d(Dst2Args p, const
             });
     } else if (warp == D2_MMA_WARP) {
         // ---- MMA issue: descriptors built once, advanced by 16-byte units ----
+        dependents_wait();              // the waits below have a limit, the kernel ahead has none
         if (lane == 0) {
             const uint64_t k16 = 256 >> 4;                  // one K step of 8 (two core matrices)
             const uint64_t d0 = sdesc(smem_u32(sm), 128, D2_SBO);
@@ -774,6 +775,7 @@ __global__ void __launch_bounds__(D2_WARPS * 32, 1) k_tc_dst2d_h(Dst2hArgs P, co
                 }
             });
     } else if (warp == D2_MMA_WARP) {
+        dependents_wait();              // the waits below have a limit, the kernel ahead has none
         if (lane == 0) {
             const uint64_t k16 = 256 >> 4;                  // one K step of 16 (two core matrices)
             const uint64_t d0 = sdesc(smem_u32(sm), 128, H_SBO);
