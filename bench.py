@@ -175,7 +175,9 @@ def stage_model(runs, prop, kin):
     The angular stage is counted as bytes when the mixed path runs it as the
     factorised tensor-core contraction (kin["tc_angular"]; the l^2 stage then
     measures ~0): psi read at every stored point in FP32 and H read and written,
-    20 bytes per stored point.  The explicit form is counted in flops."""
+    20 bytes per stored point.  The explicit form is counted in flops, and so are the
+    digit products (kin["digit_dst"], kin["digit_angular"]): the folded transforms
+    along R, and both directions of the j basis, which leave the l^2 stage empty."""
     r0 = runs[0]
     i = r0.inp
     n1, n2, na = i.npun1, i.npun2, i.nangu
@@ -190,14 +192,16 @@ def stage_model(runs, prop, kin):
         nsto += r.ntot
     ne = r0.nelec
     fused = prop.precision != "fp64" and kin["tc_angular"]
+    fold = 2.0 if kin.get("digit_dst") else 1.0
+    jbasis = kin.get("digit_angular")
     return {
         # the fused radial kernel does all four DST products in stage 0
         "dst_R": ("flop", 4.0 * rows * n2 * n2 + 4.0 * rows_sq * n2) if kin["tc_dst_fused"]
-        else ("flop", 2.0 * rows * n2 * n2),
+        else ("flop", 2.0 * rows * n2 * n2 / fold),
         "dst_r_pair": ("flop", 4.0 * rows_sq * n2),
-        "dst_R_gather": ("flop", 2.0 * rows * n2 * n2),
-        "angular": (("byte", 20.0 * nsto) if fused else ("flop", 2.0 * na * nsto)),
-        "angular_l2": ("flop", 2.0 * na * nsto * 3),
+        "dst_R_gather": ("flop", 2.0 * rows * n2 * n2 / fold),
+        "angular": (("byte", 20.0 * nsto) if fused else ("flop", (4.0 if jbasis else 2.0) * na * nsto)),
+        "angular_l2": ("flop", 0.0 if jbasis else 2.0 * na * nsto * 3),
         # FP64 path: psi_k, psi_k-1, H read, psi_k+1 written, V row, rectangle store, two
         # grid indices.  Mixed path: two grid indices, H (FP32), per source the FP32
         # potential and FP32 psi_k, psi_k-1 (FP64), psi_k+1 (FP64 and FP32), rectangle (FP32)
@@ -209,9 +213,10 @@ def stage_model(runs, prop, kin):
 
 def dominant_roofline(stages, nrec, model, kin, precision, nsto, peaks):
     """Roofline of the stage that takes the most time per iteration, against the
-    unit that executes it: the FP64 pipe (FP64 path), the tensor cores (mixed-path
-    DSTs on tcgen05), the FP32 CUDA cores (mixed-path CUDA-core DSTs and explicit
-    angular kernels) or HBM (stages counted in bytes).  stages: total ms per
+    unit that executes it: the tensor cores (mixed-path DSTs on tcgen05, exact digit
+    products of either path), the FP64 pipe (the FP64 path's other products), the FP32
+    CUDA cores (mixed-path CUDA-core DSTs and explicit angular kernels) or HBM (stages
+    counted in bytes).  stages: total ms per
     stage over nrec iterations; model: stage_model's (kind, work) per stage."""
     hbm, tf, src = peaks
     dom = max(stages, key=lambda k: stages[k])
@@ -221,17 +226,24 @@ def dominant_roofline(stages, nrec, model, kin, precision, nsto, peaks):
     traffic = None
     if precision == "mixed" and kin["tc_dst_fused"] and kin["tc_angular"] and dom in TRAFFIC_PER_POINT:
         traffic = TRAFFIC_PER_POINT[dom] * nsto
+    if kind == "flop" and kin.get("digit_dst" if dom.startswith("dst") else "digit_angular"):
+        achieved = work / t_launch / 1e12
+        return {"bound": "tensor", "achieved": achieved, "peak": tf, "unit": "TFLOP/s",
+                "frac": achieved / tf, "traffic": traffic, "kernel": dom, "peak_source": src,
+                "work": "algorithmic flops of the folded DSTs (npun2^2 along R per row, 4 nopr1^2 npun2 for the r1 "
+                        "pair) or of both directions of the j basis (4 nangu per stored point); the kernel issues %d "
+                        "FP16 products per product (base-256 digits, kind::f16 at the bf16 rate), and the peak is "
+                        "the dense bf16 one" % (28 if precision == "fp64" else 10)}
     flops = ("algorithmic flops of the stage's dense products (DST along R: 2 nopr1 npun2^2 per slab%s; "
              "r1 pair: 4 nopr1^2 npun2; explicit angular: 2 nangu per stored point, the l^2 stage for up "
              "to three coupled blocks)")
     if kind == "flop" and precision == "fp64":
-        # FP64 results, so against the FP64 pipe's nominal rate (the measured peaks hold no
-        # FP64 figure); products from exact digits on the tensor cores can pass it
+        # against the FP64 pipe's nominal rate (the measured peaks hold no FP64 figure)
         achieved = work / t_launch / 1e12
         return {"bound": "fp64", "achieved": achieved, "peak": FP64_NOMINAL_TFLOPS, "unit": "TFLOP/s",
                 "frac": achieved / FP64_NOMINAL_TFLOPS, "traffic": traffic, "kernel": dom,
                 "peak_source": "nominal GB300 FP64 rate (not measured)",
-                "work": flops % ", formed from exact digits on the tensor cores for npun2 <= 512"}
+                "work": flops % ""}
     if kind == "flop" and not on_tensor:
         achieved = work / t_launch / 1e12
         return {"bound": "fp32", "achieved": achieved, "peak": FP32_NOMINAL_TFLOPS, "unit": "TFLOP/s",
@@ -422,7 +434,7 @@ def run_gpu(args, rank, world, local):
 
     # roofline of the dominant stage, against the unit that executes it
     hbm, tf, src = load_peaks()
-    kin = out_kernels = prop.path()
+    kin = out_kernels = {**prop.path(), **{"digit_" + k: v for k, v in prop.digit_products().items()}}
     roof = dominant_roofline(stages, nrec, stage_model(runs, prop, kin), kin, args.precision, nsto,
                              (hbm, tf, src))
     # the whole iteration against HBM (the fused ideal's bytes: psi_k-1 and psi_k

@@ -149,3 +149,30 @@ def test_cpu_baseline_sample(runs):
     out = bench.cpu_baseline(bench.sample_waves([runs["tiny_j0"]]), seconds=0.5)
     assert out["kind"] == "port" and out["unit"] == "grid-pt*iter/s" and out["value"] > 0
     assert out["cores"] >= 1 and "Chebyshev iterations" in out["sample"]
+
+
+def test_roofline_of_the_digit_products():
+    """Exact digit products are charged to the tensor cores, with what they do: the folded
+    transforms and both directions of the j basis."""
+    import types
+
+    import numpy as np
+    sys.path.insert(0, ROOT)
+    import bench
+    off = dict.fromkeys(("tc_dst", "tc_dst_fused", "tc_angular", "dst_f16"), False)
+    run = types.SimpleNamespace(inp=types.SimpleNamespace(npun1=20, npun2=40, nangu=3, netot=8), ncan=2, ntot=1000, nelec=1)
+    for precision, products in (("fp64", "28 FP16"), ("mixed", "10 FP16")):
+        prop = types.SimpleNamespace(precision=precision, nflux=lambda w: 5,
+                                     tables=lambda w: {"nopr1": np.array([10, 12, 20])})
+        dense = bench.stage_model([run], prop, off)
+        digits = {**off, "digit_dst": True, "digit_angular": True}
+        model = bench.stage_model([run], prop, digits)
+        assert model["dst_R"][1] == 2 * 42 * 40 ** 2 == dense["dst_R"][1] / 2 == model["dst_R_gather"][1]
+        assert model["dst_r_pair"] == dense["dst_r_pair"]
+        assert model["angular"] == ("flop", 4.0 * 3 * 1000) and model["angular_l2"][1] == 0
+        for dom in ("dst_R", "dst_r_pair", "dst_R_gather", "angular"):
+            r = bench.dominant_roofline({dom: 5.0, "update": 1.0}, 10, model, digits, precision, 1e3, (6700.0, 1900.0, "of measured"))
+            assert r["bound"] == "tensor" and r["peak"] == 1900.0 and products in r["work"]
+            assert abs(r["achieved"] - model[dom][1] / 5e-4 / 1e12) < 1e-12
+        r = bench.dominant_roofline({"angular": 5.0}, 10, dense, {**off, "digit_dst": True}, precision, 1e3, (6700.0, 1900.0, "x"))
+        assert r["bound"] == ("fp64" if precision == "fp64" else "fp32")
