@@ -236,9 +236,6 @@ int build_device(Ctx &c)
     c.cv_pending = false;
     int na = c.na, n1 = c.n1, n2 = c.n2, ne = c.ne;
     int W = (int)c.waves.size();
-    int64_t points = 0;
-    for (auto &t : c.waves) points += t.ntot;
-    c.acc_beside = points <= (int64_t)1 << 26;
     c.ang_cw = c.k_cw > 0 ? c.k_cw : c.ang_cw_fit;
     // ---- shared grid ----
     TRY(dupload(c, &c.d_indr1, c.indr1));
@@ -776,6 +773,9 @@ int build_device(Ctx &c)
     TRY(mw3::build_tc_dst2d(c));
     TRY(mw3::build_fx_ang(c));       // smaller than the explicit matrices, so ahead of what can be given back
     TRY(mw3::build_fx(c));
+    int64_t points = 0;
+    for (auto &t : c.waves) points += t.ntot;
+    c.acc_beside = points <= (int64_t)1 << 26 || c.use_fx || c.use_fx_ang;
     c.h32 = c.use_tc_dst2d && c.use_tc_ang;
     c.d_h32 = nullptr;
     c.d_vr32 = nullptr;
@@ -1181,9 +1181,14 @@ void join_acc(Ctx &c)
 // J = 0 wave leaves most SMs idle in both, and their launches add up: mixed 256 x 128 x 60
 // took 78 us an iteration in sequence, of which the accumulators 35; beside each other 66,
 // and 53 with the programmatic launches of the H psi kernels.  Above 2^26 stored points in
-// sequence again: H psi fills the chip and loses more to the accumulators beside it than
-// they take alone.  In sequence against beside, us an iteration, mixed 256 x 128 x 60: 51.3 M
-// points 2399, 2287; 73.4 M 3342, 3350; 88.0 M 3985, 4011; 147 M 6545, 6680
+// sequence again where neither part of H psi comes from digits: the fused kernels fill the
+// chip and lose more to the accumulators beside them than these take alone.  The digit
+// kernels, one CTA an SM and bound by their MMAs, do not.  In sequence against beside, us an
+// iteration: mixed 256 x 128 x 60 51.3 M points 2414, 2297; 73.4 M 3358, 3368; 115 M 5205,
+// 5260; mixed 512 x 128 x 60 (3xTF32) 23.7 M 4985, 4927; 103 M 21056, 21234.  With digits:
+// FP64 256 x 128 x 60 39.5 M 10176, 10111; 73.4 M 18789, 18682; 166 M 42300, 42174; mixed
+// 384 x 192 x 80 75.3 M 12190, 12069; 106 M 17027, 16905; mixed 512 x 256 x 120 85.1 M 12782,
+// 12670; mixed 256 x 128 x 100 (fused DST, digit angles) 84.7 M 6537, 6473
 void run_iteration(Ctx &c)
 {
     int64_t it = c.it + 1;
