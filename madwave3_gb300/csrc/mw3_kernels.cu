@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <mutex>
 
+#include "mw3_div.cuh"
 #include "mw3_internal.h"
 #include "mw3_tc.cuh"
 
@@ -705,25 +706,6 @@ __device__ __forceinline__ void upd_fe(const UpdArgs &u, double *zf, int w, int6
         zz[0] += ck[0] * nv;
         zz[1] += ck[1] * nv;
     }
-}
-
-// a / b, correctly rounded, for a divisor that every point shares: z = 1 / b rounded
-// once on the host, then one multiply and two FMAs (Brisebarre, Muller and Raina,
-// "Accelerating correctly rounded floating-point division when the divisor is known
-// in advance", 2004).  That needs every intermediate clear of under- and overflow:
-// zdiv_ok says so for b, the exponent test for a; a zero keeps its sign, and the rest
-// (tiny, huge, infinite, NaN) is divided.  The tests are integer instructions, off
-// the FP64 pipe.
-// The FP64 update is bound by that pipe (two operations a clock an SM): a division of
-// each point took k_update 204 us an iteration at 256 x 128 x 60, J = 10 (11 blocks),
-// this 158 us, with the same bits.
-__device__ __forceinline__ double div_shared(double a, double b, double z, bool zdiv_ok)
-{
-    const unsigned hi = (unsigned)__double2hiint(a) & 0x7FFFFFFFu;
-    const double q = a * z;
-    if (zdiv_ok && hi - (200u << 20) < (1600u << 20)) return fma(fma(-q, b, a), z, q);   // 2^-823 <= |a| < 2^777
-    if (zdiv_ok && (hi | (unsigned)__double2loint(a)) == 0u) return q;
-    return a / b;
 }
 
 // one CTA per non-empty (segment, chunk) pair of the list (angles hold different
@@ -1738,7 +1720,7 @@ void launch_update(Ctx &c, int first)
     u.emindlt = c.grid.emindlt;
     u.delta2 = c.grid.delta2;
     u.rdelta = 1.0 / c.grid.delta2;
-    u.zdiv_ok = c.grid.delta2 >= 0x1p-100 && c.grid.delta2 < 0x1p100;
+    u.zdiv_ok = zdiv_ok(c.grid.delta2);
     u.r2delta = 2.0 / c.grid.delta2;
     u.vr32 = c.d_vr32;
     u.pk32 = c.d_pk32;
