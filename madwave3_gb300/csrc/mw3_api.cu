@@ -1177,7 +1177,11 @@ void join_acc(Ctx &c)
 }
 
 // one Chebyshev iteration of every wave: H psi and the update on the context's stream, the
-// accumulators beside the next iteration's H psi (in sequence while stages are timed).  One
+// accumulators beside the next iteration's H psi (in sequence while stages are timed, and in
+// the last iteration of a call, which has none to run beside: eight contexts with a call an
+// iteration and copies between share the GPU's queues; with a second stream of each in use
+// a step took 17.7 ms, without 15.3, mixed sweep J = 0..40, medians of six in one process;
+// other processes lie between 11 and 24 ms either way).  One
 // J = 0 wave leaves most SMs idle in both, and their launches add up: mixed 256 x 128 x 60
 // took 78 us an iteration in sequence, of which the accumulators 35; beside each other 66,
 // and 53 with the programmatic launches of the H psi kernels.  Above 2^26 stored points in
@@ -1189,11 +1193,11 @@ void join_acc(Ctx &c)
 // FP64 256 x 128 x 60 39.5 M 10176, 10111; 73.4 M 18789, 18682; 166 M 42300, 42174; mixed
 // 384 x 192 x 80 75.3 M 12190, 12069; 106 M 17027, 16905; mixed 512 x 256 x 120 85.1 M 12782,
 // 12670; mixed 256 x 128 x 100 (fused DST, digit angles) 84.7 M 6537, 6473
-void run_iteration(Ctx &c)
+void run_iteration(Ctx &c, bool last)
 {
     int64_t it = c.it + 1;
     const int par = (int)(it & 1);
-    const bool beside = c.side && !c.prof && c.acc_beside;
+    const bool beside = c.side && !c.prof && c.acc_beside && !last;
     hphi_all(c, c.d_pk, 0, c.G);
     if (c.nofemax > 0) mw3::launch_fe_coef(c, it);
     // psi_it overwrites psi_it-2 and its norm partials: its accumulators must be through
@@ -1207,6 +1211,8 @@ void run_iteration(Ctx &c)
         cudaEventRecord(c.ev_upd, c.stream);
         cudaStreamWaitEvent(c.side, c.ev_upd, 0);
         std::swap(c.stream, c.side);
+    } else {
+        join_acc(c);
     }
     mw3::launch_accumulators(c, it);
     mw3::launch_norms(c, c.norm_slot);
@@ -1261,7 +1267,7 @@ void capture_graph(Ctx &c, int par)
     c.capturing = true;
     c.cap_it0 = it0;
     c.cap_slot0 = slot0;
-    for (int i = 0; i < mw3::kGraphIters; i++) run_iteration(c);
+    for (int i = 0; i < mw3::kGraphIters; i++) run_iteration(c, false);
     join_acc(c);
     c.capturing = false;
     cudaError_t e = cudaStreamEndCapture(c.stream, &g);
@@ -1324,7 +1330,7 @@ int mw3_run(mw3_ctx *h, int64_t n)
                 continue;
             }
         }
-        run_iteration(c);
+        run_iteration(c, s + 1 == n);
         s++;
     }
     join_acc(c);

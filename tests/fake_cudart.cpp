@@ -13,7 +13,7 @@ namespace {
 std::mutex mu;
 std::map<void *, size_t> blocks;
 size_t used = 0, peak = 0, budget = (size_t)1 << 40;
-int regs = 96;
+int regs = 96, waits = 0;
 cudaError_t last = cudaSuccess;
 
 cudaError_t fail(cudaError_t e)
@@ -52,6 +52,12 @@ int handle;
 extern "C" {
 void fake_budget(size_t n) { budget = n; }
 void fake_registers(int n) { regs = n; }
+int fake_waits()
+{
+    const int n = waits;
+    waits = 0;
+    return n;
+}
 size_t fake_used() { return used; }
 size_t fake_peak()
 {
@@ -101,7 +107,7 @@ cudaError_t cudaGetDriverEntryPointByVersion(const char *, void **f, unsigned, u
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { return *s = reinterpret_cast<cudaStream_t>(&handle), cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return waits++, cudaSuccess; }
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaErrorNotSupported; }
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *) { return cudaErrorNotSupported; }
 cudaError_t cudaEventCreate(cudaEvent_t *e) { return *e = reinterpret_cast<cudaEvent_t>(&handle), cudaSuccess; }

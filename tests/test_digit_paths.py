@@ -129,3 +129,17 @@ def test_a_kernel_with_fewer_registers_is_left_alone(fake, shape_run, precision,
             p.close()
     finally:
         fake.fake_registers(96)
+
+
+def test_a_call_of_one_iteration_stays_on_its_stream(fake, shape_run):
+    """The accumulators run on a second stream only where another iteration of the call runs beside them."""
+    p = Propagator(shape_run(24, 40, 4, {}), "fp64")
+    p.start()
+    fake.fake_waits()
+    p.run(1)
+    assert fake.fake_waits() == 0
+    p.run(2)
+    assert fake.fake_waits() == 2            # the second stream after the first update, the first before the call's end
+    p.run(1)
+    assert fake.fake_waits() == 0
+    p.close()
