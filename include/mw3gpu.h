@@ -258,8 +258,9 @@ int mw3_kernel_launches(mw3_ctx *ctx, int64_t *count);
 #define MW3_PATH_DIGIT_ANG 128    /* the angular terms from exact base-256 digits */
 int mw3_path_flags(mw3_ctx *ctx, int32_t *flags);
 
-/* The CUDA stream (cudaStream_t) all device work of the context runs on, for
- * callers that order their own work or timing events against it. */
+/* The CUDA stream (cudaStream_t) of the context, for callers that order their
+ * own work or timing events against it.  mw3_run may use a second one inside;
+ * it starts after what is on this stream and is joined before the call returns. */
 int mw3_get_stream(mw3_ctx *ctx, void **stream);
 
 /* Per-stage timing: while enabled, mw3_run records CUDA events around each

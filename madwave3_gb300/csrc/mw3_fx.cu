@@ -58,9 +58,10 @@ struct Args {
     const T *yj;                 // [G][na][n1] yyy(j, r1) by ladder slot
     const T *l2;                 // [G][3][na][n2] xl2mat_j(Om, Om + q; R), slot q + 1, by ladder slot
     const int *cpl;              // [G][3][2]: the block Omega + q of the same wave and state, -1 where there is none
-    // [G][na] each angle's scale: its entries of the angular matrices stand x 2^sa, the vector's over it.
-    // Next to the poles every entry of a high Omega is tiny (60 angles, Omega = 10: 2e-13), and with one
-    // scale for the whole matrix it kept what it has of the 54 bits: 9e-9 of its own size there
+    // [G][na] each angle's scale: its entries of the angular matrices stand x 2^sa, the vector's
+    // over it.  Next to the poles every entry of a high Omega is tiny (60 angles, Omega = 10:
+    // 2e-13), and one scale for the whole matrix kept it to 3e-5 of itself.  Costs the angular
+    // kernels 0.1 to 1 % in FP64, 1.6 % in FP32 (384 x 192 x 80, three states: 637 -> 647 us)
     const int *sa;
     int *err;
 };

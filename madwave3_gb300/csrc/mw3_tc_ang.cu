@@ -419,8 +419,8 @@ int upload(Ctx &c, V **dst, const std::vector<V> &v)
 // Tables of the factorised angular contraction.  Returns MW3_OK with
 // c.use_tc_ang = false when the shape is outside what the kernel covers
 // (more than 64 angles or j values, a block whose j list leaves the ladder
-// j0 + k*inc, or Omega couplings that are not chain neighbours); the explicit
-// kernels then stay in use.
+// j0 + k*inc, or Omega couplings that are not chain neighbours); the digit
+// products (up to 256 angles) or the explicit kernels then run.
 int build_tc_ang(Ctx &c)
 {
     using tc::AG_K;

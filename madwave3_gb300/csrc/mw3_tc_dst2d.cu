@@ -1142,7 +1142,7 @@ std::vector<double> dst_matrix(int n);
 
 // Tables of the fused radial kernel; c.use_tc_dst2d stays false when the shape
 // is outside it (npun2 > 256 or an r1 DST length above 128: the three-kernel
-// tensor-core path or the CUDA-core path runs instead).
+// tensor-core path, the digit products or the CUDA-core path runs instead).
 int build_tc_dst2d(Ctx &c)
 {
     c.use_tc_dst2d = false;
