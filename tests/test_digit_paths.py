@@ -8,7 +8,7 @@ import subprocess
 import pytest
 
 from madwave3_gb300 import Propagator, build, propagator
-from tests.test_gpu_fx_dst import MIXED, SHAPES, SHARED
+from test_gpu_fx_dst import MIXED, SHAPES, SHARED
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 
